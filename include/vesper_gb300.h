@@ -175,13 +175,15 @@ int vesper_search(const void *spectra, const double *data, const float *vec, con
                   void *stream);
 
 /* vesper_search with explicit kernel choices, for the autotuner: HOST
- * opts[3] = {path (-1 automatic, 0 radix-stage passes, 1 register two-step
- * passes where compiled for this side and mode, 2 the fused single-kernel
+ * opts[3] = {path (-1 automatic, 0 radix-stage passes, 1 register
+ * passes where compiled for this side and mode (every side from 25 to 100), 2 the fused single-kernel
  * search where compiled, 3 pass B (x-axis DFTs, product, group sums) as
  * split-BF16 tensor-core contractions with passes A and C as path 1, else 0;
  * sides 32 and 64), channels per pass-A block (0 automatic), columns per
- * pass-B block (0 automatic)}.  Automatic picks 2, else 1, else 0.  Paths
- * 0-2 give the same results up to float32 rounding of the FFT; path 3 carries
+ * pass-B block (0 automatic); path 1 has fixed blocks and ignores the last
+ * two}.  Automatic picks 2, else 1, else 0.  Paths 0-2 give the same results
+ * up to float32 rounding of the FFT, paths 0 and 1 the same bits in most
+ * sides and modes; path 3 carries
  * the split-BF16 error (about 1e-5 of a transform's magnitude).  After a path-3
  * call, vesper_search_status reports whether a tensor-core wait timed out. */
 int vesper_search_tuned(const void *spectra, const double *data, const float *vec, const float *probs, int dim,

@@ -79,7 +79,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
                 print(r.stdout + r.stderr)
             return obj
 
-        with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+        with ThreadPoolExecutor(max_workers=min(max(8, os.cpu_count() or 8), len(srcs))) as ex:
             objs = list(ex.map(compile_one, srcs))
         tmp = LIB_PATH + f".{os.getpid()}.tmp"
         cmd = [nvcc, "-shared", "-o", tmp] + objs + ARCH

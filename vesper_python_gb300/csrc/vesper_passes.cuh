@@ -68,6 +68,7 @@ struct PassA2 {
     float2 *S;                    // [batch][nch][d][d][H]
     unsigned long long *keys;     // [nrot][nscore]
     const double *rd;             // Laplacian mode: [batch][d^3] rotated density, or null
+    const float *plain;           // Laplacian mode, register passes: [batch][d^3] filtered density
 };
 
 // Pass-A sample of rotation b of the batch: the Laplacian mode reads the
@@ -83,17 +84,6 @@ __device__ __forceinline__ void sample_a(const PassA2 &a, const float (&F)[9], i
         }
     }
     sample_fast<MODE>(a.src, F, x, y, z, out);
-}
-
-// sample_a for a side known at compile time (sample_ct in modes V/O/C/P).
-template <int MODE, int NCH, int D>
-__device__ __forceinline__ void sample_a_ct(const PassA2 &a, const float (&F)[9], int b, int x, int y, int z,
-                                            float *out) {
-    if constexpr (MODE == VESPER_MODE_VEC || MODE == VESPER_MODE_OVERLAP || MODE == VESPER_MODE_CC ||
-                  MODE == VESPER_MODE_PCC)
-        sample_ct<MODE, D>(a.src, F, x, y, z, out);
-    else
-        sample_a<MODE, NCH>(a, F, b, x, y, z, out);
 }
 
 __host__ __device__ inline size_t smem_a2(int d, int ntab, int cchunk) {

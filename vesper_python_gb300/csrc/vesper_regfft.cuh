@@ -110,6 +110,74 @@ __device__ __forceinline__ void rdft(float2 *a) {
     }
 }
 
+// ---- the same DFTs with the radix-stage passes' arithmetic ----------------------
+// Last radix of make_plan's order (4s first, then 2, 3, 5, 7, 11, 13).
+template <int N> __host__ __device__ constexpr int plan_last() {
+    for (int p : {13, 11, 7, 5, 3})
+        if (N % p == 0) return p;
+    int n = N;
+    while (n % 4 == 0) n /= 4;
+    return n == 2 ? 2 : 4;
+}
+// a * w (INV: a * conj(w)) with the fused multiply-adds spelled out in the form
+// that the radix stages' products are compiled to.
+template <bool INV>
+__device__ __forceinline__ float2 twiddle(float2 a, float2 w) {
+    const float wy = INV ? -w.y : w.y;
+    return make_float2(__fmaf_rn(a.x, w.x, -__fmul_rn(a.y, wy)), __fmaf_rn(a.y, w.x, __fmul_rn(a.x, wy)));
+}
+// An N-point DFT stage by stage as vesper_fft.cuh runs it (decimation in time,
+// the plan's radices, twiddles exp(-2 pi i m / N) = tw[TS m] from the line's own
+// table of N TS entries), so its outputs are the radix-stage passes' bit for bit.
+template <int N, bool INV, int TS>
+__device__ __forceinline__ void rdft_plan(float2 *a, const float2 *tw) {
+    if constexpr (N == 1) {
+        return;
+    } else if constexpr (plan_last<N>() == N) {
+        Dft<N, INV, float2>::run(a);
+    } else {
+        constexpr int P = plan_last<N>(), M = N / P;
+        float2 b[P][M];
+#pragma unroll
+        for (int r = 0; r < P; ++r)
+#pragma unroll
+            for (int m = 0; m < M; ++m) b[r][m] = a[r + P * m];
+#pragma unroll
+        for (int r = 0; r < P; ++r) rdft_plan<M, INV, TS * P>(b[r], tw);
+#pragma unroll
+        for (int r = 1; r < P; ++r)
+#pragma unroll
+            for (int k = 1; k < M; ++k) b[r][k] = twiddle<INV>(b[r][k], tw[TS * r * k]);
+#pragma unroll
+        for (int k = 0; k < M; ++k) {
+            float2 c[P];
+#pragma unroll
+            for (int r = 0; r < P; ++r) c[r] = b[r][k];
+            Dft<P, INV, float2>::run(c);
+#pragma unroll
+            for (int q = 0; q < P; ++q) a[k + M * q] = c[q];
+        }
+    }
+}
+
+// One step of a line FFT of length D: PFA, the register DFT above with coprime
+// factors split without twiddles, or the radix-stage passes' arithmetic.
+template <int N, int D, bool INV, bool PFA, bool LF = false>
+__device__ __forceinline__ void line_dft(float2 *a, const float2 *tw) {
+    if constexpr (PFA)
+        rdft<N, INV, LF>(a);
+    else
+        rdft_plan<N, INV, D / N>(a, tw);
+}
+// The twiddle between the two steps.
+template <bool INV, bool PFA>
+__device__ __forceinline__ float2 step_twiddle(float2 a, float2 w) {
+    if constexpr (PFA)
+        return INV ? cmulc(a, w) : cmul(a, w);
+    else
+        return twiddle<INV>(a, w);
+}
+
 // W_n^m, m < n, in shared memory (forward sign); computed per CTA.
 __device__ __forceinline__ void twiddles_n(int n, float2 *tw) {
     for (int m = threadIdx.x; m < n; m += blockDim.x) {

@@ -18,6 +18,15 @@ struct Src {
 __host__ __device__ inline int odd_up(int n) { return n | 1; }
 
 // ---- pack -------------------------------------------------------------------
+// query transforms of the scalar modes, VESPER_1_prob_new.py:548-553
+template <int MODE>
+__device__ __forceinline__ float query_value(double v, double ave) {
+    if (MODE == VESPER_MODE_OVERLAP) return v > 0 ? 1.f : 0.f;
+    if (MODE == VESPER_MODE_CC) return v > 0 ? (float)v : 0.f;
+    if (MODE == VESPER_MODE_PCC) return v > 0 ? (float)__dsub_rn(v, ave) : 0.f;
+    return 0.f;
+}
+
 template <int MODE>
 __global__ void k_pack(const double *data, const float *vec, const float *probs, int d, double ave, float4 *q4,
                        float4 *p4) {
@@ -27,17 +36,24 @@ __global__ void k_pack(const double *data, const float *vec, const float *probs,
         const float m = v != 0.0 ? 1.f : 0.f;
         float4 o;
         if (MODE == VESPER_MODE_VEC || MODE == VESPER_MODE_PROB) {
-            o = make_float4(vec[3 * i], vec[3 * i + 1], vec[3 * i + 2], m);
+            // masked voxels hold zero, so the register passes need not test the mask
+            o = m != 0.f ? make_float4(vec[3 * i], vec[3 * i + 1], vec[3 * i + 2], m) : make_float4(0.f, 0.f, 0.f, 0.f);
         } else {
-            float val = 0.f;   // query transforms, VESPER_1_prob_new.py:548-553
-            if (MODE == VESPER_MODE_OVERLAP) val = v > 0 ? 1.f : 0.f;
-            if (MODE == VESPER_MODE_CC) val = v > 0 ? (float)v : 0.f;
-            if (MODE == VESPER_MODE_PCC) val = v > 0 ? (float)__dsub_rn(v, ave) : 0.f;
-            o = make_float4(val, 0.f, 0.f, m);
+            o = make_float4(query_value<MODE>(v, ave), 0.f, 0.f, m);
         }
         q4[i] = o;
         if (MODE == VESPER_MODE_PROB) p4[i] = make_float4(probs[i], probs[n + i], probs[2 * n + i], probs[3 * n + i]);
     }
+}
+
+// The value of the scalar modes alone (4 bytes a voxel: a gather's cache lines
+// hold four times as many), for the register passes; it is zero wherever the
+// density is.
+template <int MODE>
+__global__ void k_pack_value(const double *data, int d, double ave, float *q1) {
+    const size_t n = (size_t)d * d * d;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        q1[i] = query_value<MODE>(data[i], ave);
 }
 
 // ---- gather -----------------------------------------------------------------
@@ -132,43 +148,6 @@ __device__ __forceinline__ int gather_index_fast(const float (&F)[9], int d, int
 
 template <int MODE>
 __device__ __forceinline__ void sample(const Src &s, const float *F, int x, int y, int z, float *out);
-
-// sample_fast for a side D known at compile time (modes V, O, C, P): the
-// candidate rows, the bounds and the index arithmetic fold to constants; the
-// rare multi-candidate voxels of odd sides take the general gather.  Same
-// results as sample().
-template <int MODE, int D>
-__device__ __forceinline__ void sample_ct(const Src &s, const float (&F)[9], int x, int y, int z, float *out) {
-    static_assert(MODE == VESPER_MODE_VEC || MODE == VESPER_MODE_OVERLAP || MODE == VESPER_MODE_CC ||
-                  MODE == VESPER_MODE_PCC, "sample_ct: modes V, O, C, P");
-    const int ix = cand1(x, D), iy = cand1(y, D), iz = cand1(z, D);
-    bool hit = false;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if ((ix | iy | iz) < 0) {
-        if (ix == -2 || iy == -2 || iz == -2) {
-            if (ix != -1 && iy != -1 && iz != -1) {
-                sample<MODE>(s, F, x, y, z, out);
-                return;
-            }
-        }
-    } else {
-        constexpr float hc = 0.5f * (float)D;
-        int ox, oy, oz;
-        if (old_index(F, D, hc, (float)ix - hc, (float)iy - hc, (float)iz - hc, ox, oy, oz)) {
-            v = __ldg(s.q4 + (ox * D + oy) * D + oz);
-            hit = v.w != 0.f;
-        }
-    }
-    if (MODE == VESPER_MODE_VEC) {
-        float r[3] = {0.f, 0.f, 0.f};
-        if (hit) rotate_vec(F, v.x, v.y, v.z, r);
-        out[0] = r[0];
-        out[1] = r[1];
-        out[2] = r[2];
-    } else {
-        out[0] = hit ? v.x : 0.f;
-    }
-}
 
 // Channel values of the rotated query at (x, y, z), rotation matrix in
 // registers; same results as sample().

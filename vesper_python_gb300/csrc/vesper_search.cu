@@ -34,8 +34,14 @@ struct SearchCfg {
     int path;   // 0: radix-stage passes, 1: register two-step passes
 };
 
-// ---- register two-step passes: the sides compiled in (vesper_regsearch_*.cu)
-const RegEntry *find_reg(int mode, int d);
+// ---- register passes: the sides and modes compiled in (vesper_sides_*.cu)
+static const RegEntry *find_reg(int mode, int d) {
+    using Find = const RegEntry *(*)(int, int);
+    const int kind = reg_kind(mode);
+    for (Find f : {find_reg_pfa_a, find_reg_pfa_b, find_reg_a, find_reg_b, find_reg_c, find_reg_d, find_reg_e, find_reg_f, find_reg_g, find_reg_h, find_reg_i, find_reg_j, find_reg_k, find_reg_l})
+        if (const RegEntry *e = f(d, kind)) return e;
+    return nullptr;
+}
 
 // vesper_fused.cu: 1 if a fused single-kernel search is compiled for (mode,
 // side) -- launched when rc is non-null, its status stored there -- else 0.
@@ -107,6 +113,12 @@ static void launch_pack(const double *data, const float *vec, const float *probs
     k_pack<MODE><<<blocks, 256, 0, st>>>(data, vec, probs, d, ave, q4, p4);
 }
 
+template <int MODE>
+static void launch_pack_value(const double *data, int d, double ave, float4 *q4, cudaStream_t st) {
+    const size_t n = (size_t)d * d * d;
+    k_pack_value<MODE><<<(int)std::min<size_t>((n + 255) / 256, 152 * 8), 256, 0, st>>>(data, d, ave, (float *)q4);
+}
+
 }  // namespace vg
 
 using namespace vg;
@@ -130,21 +142,31 @@ extern "C" int vesper_search_nscore(int mode, int with_mix) {
 }
 
 // Laplacian mode: the rotated density of every rotation of a batch
-// (rot_mrc's gather, density != 0 mask), so that pass A computes the filter
-// from plain reads instead of seven gathers per voxel.
+// (rot_mrc's gather, density != 0 mask), so that the filter is computed from
+// plain reads instead of seven gathers per voxel.  A voxel with one candidate
+// row per axis needs no mask: a masked density is zero.
 __global__ void k_rot_density(const Src s, const float *rotmats, int r0, double *rd) {
-    __shared__ float F[9];
-    const int b = blockIdx.y;
-    if (threadIdx.x < 9) F[threadIdx.x] = rotmats[(size_t)(r0 + b) * 9 + threadIdx.x];
-    __syncthreads();
-    const int d = s.d;
-    const size_t n = (size_t)d * d * d;
-    const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = blockIdx.y, d = s.d;
+    float F[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) F[i] = __ldg(rotmats + (size_t)(r0 + b) * 9 + i);
+    const int n = d * d * d, v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n) return;
-    const int x = (int)(v / ((size_t)d * d)), y = (int)((v / d) % d), z = (int)(v % d);
-    float4 w;
-    const int i = gather4(F, d, x, y, z, s.q4, w);
+    const int x = v / (d * d), y = (v / d) % d, z = v % d;
+    int i = gather_index_fast(F, d, x, y, z);
+    if (i == -2) {
+        float4 w;
+        i = gather4(F, d, x, y, z, s.q4, w);
+    }
     rd[(size_t)b * n + v] = i >= 0 ? s.data[i] : 0.0;
+}
+
+// laplacian_filter of the rotated densities, for the register passes.
+__global__ void k_laplace(const double *rd, int d, float *out) {
+    const int n = d * d * d, v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    const size_t o = (size_t)blockIdx.y * n;
+    out[o + v] = lap_from_rd(rd + o, d, v / (d * d), (v / d) % d, v % d);
 }
 
 extern "C" int vesper_search_workspace_size(int dim, int mode, int batch, int nrot, size_t *bytes) {
@@ -186,33 +208,19 @@ static int search_impl(const void *spectra, const double *data, const float *vec
     if (!plan_passes(dim, mode, P, &cfg))
         return fail(VESPER_ERR_UNSUPPORTED, "grid side %d does not fit shared memory", dim);
     cfg.path = 0;
-    const RegEntry *reg = find_reg(mode, dim);
     const int want_path = opts ? opts[0] : -1;
+    // fused single-kernel search where it is compiled for (mode, side)
+    const bool fused = (want_path == 2 || want_path < 0) &&
+                       vesper_fused_search(mode, dim, Src{}, nullptr, nullptr, 0, 1, nullptr, nullptr, nullptr) != 0;
+    if (want_path == 2 && !fused)
+        return fail(VESPER_ERR_UNSUPPORTED, "no fused search compiled for mode %d, side %d", mode, dim);
+    const RegEntry *reg = fused ? nullptr : find_reg(mode, dim);
     // path 3: pass B on the tensor cores (split-BF16), passes A and C as path 1 (else 0)
     const bool tcb = want_path == 3;
     if (tcb && !tc_pass_b_supported(dim))
         return fail(VESPER_ERR_UNSUPPORTED, "tensor-core pass B: side %d (32 and 64 only)", dim);
     if (reg && want_path != 0) {
-        const size_t lim = (size_t)smem_limit();
-        const int nchr = mode_nch(mode), ngrr = mode_ngrp(mode);
-        int cc = 0, W = 0;
-        for (size_t cap : {lim / 2 - 1024, lim}) {
-            for (int c = nchr; c >= 1 && !cc; --c)
-                if (reg->sa(c) <= cap) cc = c;
-            if (cc) break;
-        }
-        for (int w : {32, 16, 8, 4, 2, 1})
-            if (!W && reg->sb(nchr, ngrr, w) <= lim / 2 - 1024) W = w;
-        if (opts && opts[1] > 0 && opts[1] <= nchr && reg->sa(opts[1]) <= lim) cc = opts[1];
-        if (opts && opts[2] > 0 && reg->sb(nchr, ngrr, opts[2]) <= lim) W = opts[2];
-        if (cc && W && reg->sc(ngrr) <= lim) {
-            cfg.path = 1;
-            cfg.cchunk = cc;
-            cfg.W = W;
-            cfg.sa = reg->sa(cc);
-            cfg.sb = reg->sb(nchr, ngrr, W);
-            cfg.sc = reg->sc(ngrr);
-        }
+        cfg.path = 1;
     } else if (opts) {
         const int nchr = mode_nch(mode), ngrr = mode_ngrp(mode);
         const size_t lim = (size_t)smem_limit();
@@ -246,7 +254,15 @@ static int search_impl(const void *spectra, const double *data, const float *vec
     unsigned long long *keys = cv.take<unsigned long long>((size_t)nrot * 3);
     double *rd = mode == VESPER_MODE_LAPLACIAN ? cv.take<double>((size_t)batch * N) : nullptr;
 
-    switch (mode) {
+    const bool values = !fused && cfg.path == 1;   // the register passes take the scalar modes as plain values
+    switch (values ? mode : mode + 16) {
+        case VESPER_MODE_OVERLAP: launch_pack_value<VESPER_MODE_OVERLAP>(data, dim, ave, q4, st); break;
+        case VESPER_MODE_CC: launch_pack_value<VESPER_MODE_CC>(data, dim, ave, q4, st); break;
+        case VESPER_MODE_PCC: launch_pack_value<VESPER_MODE_PCC>(data, dim, ave, q4, st); break;
+        default: break;
+    }
+    const bool packed = values && (mode == VESPER_MODE_OVERLAP || mode == VESPER_MODE_CC || mode == VESPER_MODE_PCC);
+    switch (packed ? -1 : mode) {
         case VESPER_MODE_VEC: launch_pack<VESPER_MODE_VEC>(data, vec, probs, dim, ave, q4, p4, st); break;
         case VESPER_MODE_OVERLAP: launch_pack<VESPER_MODE_OVERLAP>(data, vec, probs, dim, ave, q4, p4, st); break;
         case VESPER_MODE_CC: launch_pack<VESPER_MODE_CC>(data, vec, probs, dim, ave, q4, p4, st); break;
@@ -265,13 +281,16 @@ static int search_impl(const void *spectra, const double *data, const float *vec
         mx.pstd = (float)mix[3];
         mx.pave = (float)mix[4];
     }
-    PassA2 pa{Src{q4, p4, data, dim}, rotmats, 0, nch, cfg.cchunk, nscore, P, S, keys, rd};
+    PassA2 pa{Src{q4, p4, data, dim}, rotmats, 0, nch, cfg.cchunk, nscore, P, S, keys, rd, (const float *)U};
     PassB2 pb{S, (const float2 *)spectra, U, dim, nch, ngrp, mode == VESPER_MODE_PROB ? 3 : nch, cfg.W, P};
     PassC2 pc{U, dim, ngrp, 0, nscore, P, mx, keys};
-    allow_smem(k_pass_b, cfg.sb);
-    allow_smem(k_pass_c<1>, cfg.sc);
-    allow_smem(k_pass_c<2>, cfg.sc);
-    allow_smem(k_pass_c<3>, cfg.sc);
+    if (!fused && cfg.path == 0) {
+        allow_smem(k_pass_b, cfg.sb);
+        allow_smem(k_pass_c<1>, cfg.sc);
+        allow_smem(k_pass_c<2>, cfg.sc);
+        allow_smem(k_pass_c<3>, cfg.sc);
+    }
+    const int kind = reg_kind(mode);
     const int nbx = (dim * H + cfg.W - 1) / cfg.W;
     int slot = 0;
     auto drain = [&](int sl) {
@@ -290,21 +309,14 @@ static int search_impl(const void *spectra, const double *data, const float *vec
         cudaEventRecord(tm->ev[slot][pass][edge], st);
         if (edge == 1) tm->used[slot][pass] = true;
     };
-    // fused single-kernel search where it is compiled for (mode, side)
-    bool fused = false;
-    if (want_path == 2 || want_path < 0) {
+    if (fused) {
         int frc = VESPER_OK;
         mark(0, 0);
-        fused = vesper_fused_search(mode, dim, Src{q4, p4, data, dim}, rotmats, spectra, nrot, nscore, keys, st,
-                                    &frc) != 0;
-        if (fused && frc) return frc;
-        if (fused) {
-            mark(0, 1);
-            slot = (slot + 1) % kRing;
-        }
+        vesper_fused_search(mode, dim, Src{q4, p4, data, dim}, rotmats, spectra, nrot, nscore, keys, st, &frc);
+        if (frc) return frc;
+        mark(0, 1);
+        slot = (slot + 1) % kRing;
     }
-    if (want_path == 2 && !fused)
-        return fail(VESPER_ERR_UNSUPPORTED, "no fused search compiled for mode %d, side %d", mode, dim);
     for (int r0 = 0; !fused && r0 < nrot; r0 += batch) {
         const int nb = std::min(batch, nrot - r0);
         pa.r0 = r0;
@@ -316,21 +328,25 @@ static int search_impl(const void *spectra, const double *data, const float *vec
             VG_CHECK_LAUNCH("k_rot_density");
         }
         if (cfg.path == 1) {
-            reg->a(gplane, kThreads, cfg.sa, st, pa);
-            VG_CHECK_LAUNCH("k_rpass_a");
+            if (rd) {   // into the U region, which pass B writes only after pass A has read it
+                k_laplace<<<dim3((unsigned)((N + 255) / 256), nb), 256, 0, st>>>(rd, dim, (float *)U);
+                VG_CHECK_LAUNCH("k_laplace");
+            }
+            reg->a[kind](nb, st, pa);
+            VG_CHECK_LAUNCH("register pass A");
             mark(0, 1);
             mark(1, 0);
             if (tcb) {
                 rc = tc_pass_b(pb, nb, status, st);
                 if (rc) return rc;
             } else {
-                reg->b(dim3(nbx, nb), kThreads, cfg.sb, st, pb);
-                VG_CHECK_LAUNCH("k_rpass_b");
+                reg->b[kind](nb, st, pb);
+                VG_CHECK_LAUNCH("register pass B");
             }
             mark(1, 1);
             mark(2, 0);
-            reg->c(gplane, kThreads, cfg.sc, st, pc, nscore);
-            VG_CHECK_LAUNCH("k_rpass_c");
+            reg->c[kind](nb, st, pc);
+            VG_CHECK_LAUNCH("register pass C");
             mark(2, 1);
             slot = (slot + 1) % kRing;
             continue;
@@ -448,8 +464,8 @@ extern "C" int vesper_search_plan(int dim, int mode, int batch, int nrot, const 
     }
     const int nb = nrot > 0 ? (nrot + batch - 1) / batch : 0;
     *path_out = path;
-    // pack + passes (+ the gathered density of each Laplacian batch) + decode
-    *launches_out = nrot > 0 ? 2 + (path == 2 ? 1 : (mode == VESPER_MODE_LAPLACIAN ? 4 : 3) * nb) : 0;
+    // pack + passes (+ each Laplacian batch's gathered and filtered density) + decode
+    *launches_out = nrot > 0 ? 2 + (path == 2 ? 1 : (mode != VESPER_MODE_LAPLACIAN ? 3 : path ? 5 : 4) * nb) : 0;
     return VESPER_OK;
 }
 

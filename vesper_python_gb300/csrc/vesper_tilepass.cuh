@@ -1,0 +1,541 @@
+// Search passes for grid sides d = N1 * N2 above the whole-line kernels' range
+// (vesper_regpass.cuh): every line FFT runs as two register steps (of N1 and of
+// N2 points), the steps of a line meeting in shared memory.
+//
+//   A  one x plane per CTA.  The CTA gathers the plane; each warp then owns tiles of
+//      4 packed z lines (8 rows), which it transforms along z and unpacks into rows
+//      with warp barriers only; then the block transforms the columns along y,
+//      straight to S.
+//   B  W spectrum columns per CTA, several rotations one after another: the
+//      columns' target values stay in registers for all of them.
+//   C  one x plane per CTA: inverse y in place, then each warp owns PL row
+//      pairs for the inverse z transform and the argmax.
+//
+// Inputs, outputs and layouts are those of the radix-stage passes.  Two kinds of
+// arithmetic: the radix-stage passes' own, bit for bit (the general form), or line
+// DFTs whose coprime factors split without twiddles (PFA) with the inverse's
+// steps in the opposite order.
+//
+// What bounds them (GB300, mode V, microseconds per rotation A / B / C, against
+// the kernels they replace): side 75 3.14 / 1.52 / 0.99 (one block-wide step after
+// another, general gather in line: 5.41 / 1.74 / 1.04), side 48 0.89 / 0.67 / 0.30
+// (radix stages 2.26 / 1.60 / 1.06), side 80 3.73 / 2.4 / 1.14 (11.9 / 7.4 / 3.1),
+// prob mode at side 64 6.4 / 3.4 / 2.7 (18.0 / 5.4 / 2.7).  A is bound by issue
+// slots and shared-memory wavefronts together (56 % and 58 % at 15 warps per SM;
+// one warp per tile gives 30): strides without bank conflicts took side 75 from
+// 4.17 to 3.93, one warp per tile within 64 registers to 3.48, and the middle
+// voxels of odd sides, loaded together and shared out over the CTA, to 3.14.  B is
+// bound by the S and T it reads: T from L2 once per 8 rotations instead of once
+// each took side 75 from 1.74 to 1.52.
+#pragma once
+
+#include "vesper_regfft.cuh"
+#include "vesper_tilegather.cuh"
+
+namespace vg {
+
+// Shared-memory layout of a plane.  A 64-bit access is conflict-free when the 16
+// lanes of a half warp fall in 16 different 8-byte banks.  With the row stride RS
+// = 2 mod 4, four consecutive packed lines (stride LS = 2 RS) start 4 banks
+// apart, so lanes that run over 4 lines and then over 4 consecutive elements cover
+// all 16; between the steps element (k1, j2) of a line sits at P2 k1 + j2 with P2
+// odd, so that runs over k1 do the same; CS = N2 mod 4 continues the pattern
+// from one channel to the next.
+constexpr int up_to_mod(int n, int mod, int rem) { return n + ((rem - n) % mod + mod) % mod; }
+// SPLIT: a line's elements lie half in its first row's storage, half in its second's.
+template <int N1, int N2, bool SPLIT = false>
+struct TGeom {
+    static constexpr int D = N1 * N2, H = D / 2 + 1, NP = (D + 1) / 2;
+    static constexpr int P2 = N2 | 1;
+    static constexpr int kHalf = SPLIT ? (N1 + 1) / 2 * P2 : (N1 * P2 + 1) / 2;
+    static constexpr int RS = up_to_mod(H > kHalf ? H : kHalf, 4, 2);   // row stride
+    static constexpr int LS = 2 * RS;          // packed line p lives in rows 2p and 2p + 1
+    static constexpr int CS = up_to_mod(NP * LS, 4, N2 % 4);   // channel stride
+    static constexpr int TP = (NP + 3) / 4;    // gather tiles of 4 lines
+    // where element z = j2 + N2 j1 of a line waits for step 1
+    static __device__ __forceinline__ int pos(int z) { return P2 == N2 ? z : z / N2 * P2 + z % N2; }
+};
+
+// ---- pass A -------------------------------------------------------------------
+template <int SRC, int N1, int N2>
+__host__ __device__ constexpr size_t smem_ta() {
+    using G = TGeom<N1, N2>;
+    return (size_t)((G::D + 1) / 2 * 2) * sizeof(float2) + (size_t)src_nch<SRC>() * G::CS * sizeof(float2);
+}
+
+// Warps per CTA: one per 4-line tile.  Resident CTAs the register budget is
+// sized for: as many as shared memory allows, with at least 64 registers a thread.
+template <int N1, int N2> __host__ __device__ constexpr int ta_warps() { return TGeom<N1, N2>::TP; }
+template <int SRC, int N1, int N2> __host__ __device__ constexpr int ta_ctas() {
+    constexpr int by_smem = (int)((228 * 1024) / (smem_ta<SRC, N1, N2>() + 1024));
+    constexpr int by_regs = 65536 / (64 * ta_warps<N1, N2>() * 32);
+    return by_smem < by_regs ? by_smem : by_regs;
+}
+
+template <int SRC, int N1, int N2, bool PFA>
+__device__ __forceinline__ void tpass_a(const PassA2 &a, int c0) {
+    using G = TGeom<N1, N2>;
+    constexpr int D = G::D, H = G::H, NP = G::NP, RS = G::RS, LS = G::LS, CS = G::CS, P2 = G::P2, NCH = src_nch<SRC>();
+    constexpr int NW = ta_warps<N1, N2>();
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int x = blockIdx.x, b = blockIdx.y, r = a.r0 + b;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2 *twn = (float2 *)smem;
+    float2 *buf = twn + (D + 1) / 2 * 2;   // [NCH][NP][LS]
+    twiddles_n(D, twn);
+    if (x == 0 && c0 == 0 && threadIdx.x < a.nscore) a.keys[(size_t)r * a.nscore + threadIdx.x] = 0ull;
+    float F[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) F[i] = __ldg(a.rotmats + (size_t)r * 9 + i);
+    gather_plane<SRC, D, LS, CS, NW>(a, F, b, x, buf, [](int z) { return G::pos(z); });
+    __syncthreads();
+    for (int pt = warp; pt < G::TP; pt += NW) {
+        // z step 1, in place: items (c, j2, line), line fastest
+        for (int it = lane; it < NCH * 4 * N2; it += 32) {
+            const int p = pt * 4 + (it & 3), j2 = (it >> 2) % N2, c = (it >> 2) / N2;
+            if (p < NP) {
+                float2 *line = buf + c * CS + p * LS + j2;
+                float2 v[N1];
+#pragma unroll
+                for (int j1 = 0; j1 < N1; ++j1) v[j1] = line[P2 * j1];
+                line_dft<N1, D, false, PFA>(v, twn);
+#pragma unroll
+                for (int k1 = 0; k1 < N1; ++k1) line[P2 * k1] = (k1 && j2) ? step_twiddle<false, PFA>(v[k1], twn[j2 * k1]) : v[k1];
+            }
+        }
+        __syncwarp();
+        // z step 2 and unpack into the line's own two rows: items (line, q), q
+        // in [0, N1/2], whole lines per round, read before they are written
+        constexpr int NQ = N1 / 2 + 1, LPR = 32 / NQ;
+        const int lq = lane % LPR, q = lane / LPR, q2 = (N1 - q) % N1;   // line fastest
+#pragma unroll 1
+        for (int l0 = 0; l0 < NCH * 4; l0 += LPR) {
+            const int l = l0 + lq, p = pt * 4 + (l & 3), c = l >> 2;
+            const bool on = q < NQ && l < NCH * 4 && p < NP;
+            float2 *line = buf + c * CS + p * LS;
+            float2 u[N2], w2[N2];
+            if (on) {
+#pragma unroll
+                for (int j2 = 0; j2 < N2; ++j2) u[j2] = line[P2 * q + j2];
+#pragma unroll
+                for (int j2 = 0; j2 < N2; ++j2) w2[j2] = line[P2 * q2 + j2];
+                line_dft<N2, D, false, PFA>(u, twn);
+                line_dft<N2, D, false, PFA>(w2, twn);
+            }
+            __syncwarp();
+            if (on) {
+                float2 *row0 = line, *row1 = line + RS;
+#pragma unroll
+                for (int k2 = 0; k2 < N2; ++k2) {
+                    const int k = q + N1 * k2;
+                    if (k < H) {
+                        float2 A, B;
+                        unpack_pair(u[k2], (q == 0) ? u[(N2 - k2) % N2] : w2[N2 - 1 - k2], A, B);
+                        row0[k] = A;
+                        row1[k] = B;
+                    }
+                    const int kb = q2 + N1 * k2;
+                    if (q != 0 && q2 != q && kb < H) {
+                        float2 A, B;
+                        unpack_pair(w2[k2], u[N2 - 1 - k2], A, B);
+                        row0[kb] = A;
+                        row1[kb] = B;
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+    // y step 1, in place: items (c, j2, kz), kz fastest
+    for (int t = threadIdx.x; t < NCH * N2 * H; t += NW * 32) {
+        const int kz = t % H, cj = t / H, j2 = cj % N2, c = cj / N2;
+        float2 *col = buf + c * CS + j2 * RS + kz;
+        float2 v[N1];
+#pragma unroll
+        for (int j1 = 0; j1 < N1; ++j1) v[j1] = col[N2 * j1 * RS];
+        line_dft<N1, D, false, PFA>(v, twn);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1) col[N2 * k1 * RS] = (k1 && j2) ? step_twiddle<false, PFA>(v[k1], twn[j2 * k1]) : v[k1];
+    }
+    __syncthreads();
+    // y step 2: items (c, k1, kz), kz fastest -> S rows ky = k1 + N1 k2
+    float2 *out = a.S + (((size_t)b * a.nch + c0) * D + x) * (size_t)(D * H);
+    for (int t = threadIdx.x; t < NCH * N1 * H; t += NW * 32) {
+        const int kz = t % H, ck = t / H, k1 = ck % N1, c = ck / N1;
+        const float2 *col = buf + c * CS + N2 * k1 * RS + kz;
+        float2 u[N2];
+#pragma unroll
+        for (int j2 = 0; j2 < N2; ++j2) u[j2] = col[j2 * RS];
+        line_dft<N2, D, false, PFA>(u, twn);
+        float2 *dst = out + (size_t)c * (D * D * H) + k1 * H + kz;
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) dst[N1 * k2 * H] = u[k2];
+    }
+}
+
+template <int SRC, int N1, int N2, bool PFA>
+__global__ void __launch_bounds__(ta_warps<N1, N2>() * 32, ta_ctas<SRC, N1, N2>()) k_tpass_a(const PassA2 a) {
+    tpass_a<SRC, N1, N2, PFA>(a, 0);
+}
+// prob mode: the vector channels and the probability channels in CTAs of their own
+template <int N1, int N2, bool PFA>
+__global__ void __launch_bounds__(ta_warps<N1, N2>() * 32, ta_ctas<kSrcProb, N1, N2>()) k_tpass_a_prob(const PassA2 a) {
+    if (blockIdx.z == 0)
+        tpass_a<kSrcVec, N1, N2, PFA>(a, 0);
+    else
+        tpass_a<kSrcProb, N1, N2, PFA>(a, 3);
+}
+
+// ---- pass B -------------------------------------------------------------------
+template <int N1> __host__ __device__ constexpr int tb_cols() { return N1 >= 9 ? 16 : 32; }
+template <int N1> __host__ __device__ constexpr int tb_threads() { return (N1 * tb_cols<N1>() + 31) / 32 * 32; }
+// Rotations side by side in a CTA: one channel alone leaves most threads of steps 1 and 3 idle.
+template <int NCH> __host__ __device__ constexpr int tb_side() { return NCH == 1 ? 3 : 1; }
+template <int NCH, int N1, int N2>
+__host__ __device__ constexpr size_t smem_tb() {
+    return (size_t)((N1 * N2 + 1) / 2 * 2) * sizeof(float2) +
+           (size_t)tb_side<NCH>() * (NCH + 1) * N1 * N2 * tb_cols<N1>() * sizeof(float2);
+}
+
+template <int NCH, int N1, int N2, bool PFA>
+__device__ __forceinline__ void tpass_b(const PassB2 &a, int c0, int grp, int nb, int rper) {
+    constexpr int D = N1 * N2, H = D / 2 + 1, dH = D * H, W = tb_cols<N1>(), TB = tb_threads<N1>();
+    constexpr int NR = tb_side<NCH>();
+    extern __shared__ __align__(16) unsigned char smem[];
+    float2 *twn = (float2 *)smem;
+    float2 *buf = twn + (D + 1) / 2 * 2;              // [NR][NCH][D][W]
+    float2 *pbuf = buf + (size_t)NR * NCH * D * W;    // [NR][D][W]
+    const int j0 = blockIdx.x * W, b0 = blockIdx.y * rper, b1 = min(nb, b0 + rper);
+    twiddles_n(D, twn);
+    // the thread's target values: item (k1, w) of step 2, for every rotation
+    const int w2 = threadIdx.x % W, k1_ = threadIdx.x / W;
+    const bool on2 = threadIdx.x < N1 * W && j0 + w2 < dH;
+    float2 tv[NCH][N2];
+#pragma unroll
+    for (int c = 0; c < NCH; ++c)
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2)
+            tv[c][k2] = on2 ? __ldg(a.T + (size_t)(c0 + c) * D * dH + (size_t)(k1_ + N1 * k2) * dH + j0 + w2)
+                            : make_float2(0.f, 0.f);
+    __syncthreads();
+    for (int b = b0; b < b1; b += NR) {
+        const float2 *src = a.S + ((size_t)b * a.nch + c0) * D * dH + j0;
+        // forward step 1: items (rotation, c, j2, w) from global
+        for (int t = threadIdx.x; t < NR * NCH * N2 * W; t += TB) {
+            const int w = t % W, cj = t / W, j2 = cj % N2, rc = cj / N2, c = rc % NCH, rr = rc / NCH;
+            float2 v[N1];
+            const float2 *s = src + ((size_t)(rr * a.nch + c) * D + j2) * dH + w;
+            const bool on = j0 + w < dH && (NR == 1 || b + rr < b1);
+#pragma unroll
+            for (int j1 = 0; j1 < N1; ++j1) v[j1] = on ? s[(size_t)(N2 * j1) * dH] : make_float2(0.f, 0.f);
+            line_dft<N1, D, false, PFA>(v, twn);
+            float2 *col = buf + (size_t)(rc * D + j2) * W + w;
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) col[N2 * k1 * W] = (k1 && j2) ? step_twiddle<false, PFA>(v[k1], twn[j2 * k1]) : v[k1];
+        }
+        __syncthreads();
+        // forward step 2, product with conj(T), channel sum; PFA: inverse step 2 with
+        // conjugate twiddles into pbuf rows k1 + N1 j2, else the sums themselves there
+        if (threadIdx.x < N1 * W) {
+#pragma unroll
+            for (int rr = 0; rr < NR; ++rr) {
+                float2 acc[N2];
+#pragma unroll
+                for (int k2 = 0; k2 < N2; ++k2) acc[k2] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int c = 0; c < NCH; ++c) {
+                    const float2 *col = buf + (size_t)((rr * NCH + c) * D + N2 * k1_) * W + w2;
+                    float2 u[N2];
+#pragma unroll
+                    for (int j2 = 0; j2 < N2; ++j2) u[j2] = col[j2 * W];
+                    line_dft<N2, D, false, PFA>(u, twn);
+#pragma unroll
+                    for (int k2 = 0; k2 < N2; ++k2) acc[k2] = cadd(acc[k2], cmul(tv[c][k2], u[k2]));
+                }
+                if constexpr (PFA) rdft<N2, true>(acc);
+                float2 *col = pbuf + (rr * D + k1_) * W + w2;
+#pragma unroll
+                for (int j2 = 0; j2 < N2; ++j2)
+                    col[N1 * j2 * W] = (PFA && k1_ && j2) ? cmulc(acc[j2], twn[j2 * k1_]) : acc[j2];
+            }
+        }
+        __syncthreads();
+        float2 *dst = a.U + ((size_t)b * a.ngrp + grp) * D * dH + j0;
+        if constexpr (!PFA) {
+            // inverse steps in the forward's order: step 1 in place, items (rotation,
+            // j2, w); step 2, items (rotation, k1, w) -> U rows x = k1 + N1 k2
+            for (int t = threadIdx.x; t < NR * N2 * W; t += TB) {
+                const int w = t % W, rj = t / W, j2 = rj % N2, rr = rj / N2;
+                float2 *col = pbuf + (rr * D + j2) * W + w;
+                float2 v[N1];
+#pragma unroll
+                for (int j1 = 0; j1 < N1; ++j1) v[j1] = col[N2 * j1 * W];
+                rdft_plan<N1, true, N2>(v, twn);
+#pragma unroll
+                for (int k1 = 0; k1 < N1; ++k1) col[N2 * k1 * W] = (k1 && j2) ? twiddle<true>(v[k1], twn[j2 * k1]) : v[k1];
+            }
+            __syncthreads();
+            if (threadIdx.x < N1 * W) {
+#pragma unroll
+                for (int rr = 0; rr < NR; ++rr) {
+                    const float2 *col = pbuf + (rr * D + N2 * k1_) * W + w2;
+                    float2 u[N2];
+#pragma unroll
+                    for (int j2 = 0; j2 < N2; ++j2) u[j2] = col[j2 * W];
+                    rdft_plan<N2, true, N1>(u, twn);
+                    if (on2 && (NR == 1 || b + rr < b1))
+#pragma unroll
+                        for (int k2 = 0; k2 < N2; ++k2)
+                            dst[((size_t)rr * a.ngrp * D + k1_ + N1 * k2) * dH + w2] = u[k2];
+                }
+            }
+            continue;
+        }
+        // inverse step 1: items (rotation, j2, w) -> U rows x = j2 + N2 j1
+        for (int t = threadIdx.x; t < NR * N2 * W; t += TB) {
+            const int w = t % W, rj = t / W, j2 = rj % N2, rr = rj / N2;
+            const float2 *col = pbuf + (rr * D + N1 * j2) * W + w;
+            float2 v[N1];
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) v[k1] = col[k1 * W];
+            rdft<N1, true>(v);
+            if (j0 + w < dH && (NR == 1 || b + rr < b1))
+#pragma unroll
+                for (int j1 = 0; j1 < N1; ++j1)
+                    dst[((size_t)rr * a.ngrp * D + j2 + N2 * j1) * dH + w] = v[j1];
+        }
+    }
+}
+
+template <int NCH, int N1, int N2, bool PFA>
+__global__ void __launch_bounds__(tb_threads<N1>()) k_tpass_b(const PassB2 a, int nb, int rper) {
+    tpass_b<NCH, N1, N2, PFA>(a, 0, 0, nb, rper);
+}
+template <int N1, int N2, bool PFA>
+__global__ void __launch_bounds__(tb_threads<N1>()) k_tpass_b_prob(const PassB2 a, int nb, int rper) {
+    if (blockIdx.z == 0)
+        tpass_b<3, N1, N2, PFA>(a, 0, 0, nb, rper);
+    else
+        tpass_b<4, N1, N2, PFA>(a, 3, 1, nb, rper);
+}
+
+// ---- pass C -------------------------------------------------------------------
+template <int N1, int N2> __host__ __device__ constexpr int tc_warps() { return N1 * N2 <= 32 ? 2 : N1 * N2 <= 48 ? 4 : 8; }
+template <int NGRP, int N1, int N2, bool PFA>
+__host__ __device__ constexpr size_t smem_tc() {
+    using G = TGeom<N1, N2, !PFA>;
+    return (size_t)((G::D + 1) / 2 * 2) * sizeof(float2) + (size_t)NGRP * G::CS * sizeof(float2) +
+           3 * 8 * sizeof(unsigned long long);
+}
+
+template <int NGRP, int SC, int N1, int N2, bool PFA>
+__global__ void __launch_bounds__(tc_warps<N1, N2>() * 32) k_tpass_c(const PassC2 a) {
+    using G = TGeom<N1, N2, !PFA>;
+    constexpr int D = G::D, H = G::H, NP = G::NP, RS = G::RS, LS = G::LS, CS = G::CS, P2 = G::P2;
+    constexpr int NW = tc_warps<N1, N2>(), PL = (NP + NW - 1) / NW;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int x = blockIdx.x, b = blockIdx.y, r = a.r0 + b;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2 *twn = (float2 *)smem;
+    float2 *buf = twn + (D + 1) / 2 * 2;   // [NGRP][2 NP][RS]
+    unsigned long long *red = (unsigned long long *)(buf + NGRP * CS);
+    twiddles_n(D, twn);
+    __syncthreads();
+    const float2 *src0 = a.U + ((size_t)b * NGRP * D + x) * (size_t)(D * H);
+    if constexpr (!PFA) {
+        // inverse y in the forward's order.  Step 1 from U: items (g, j2, kz) -> rows
+        // N2 k1 + j2; step 2, in place: items (g, k1, kz), row y = k1 + N1 k2 stays at
+        // N2 k1 + k2
+        for (int t = threadIdx.x; t < NGRP * N2 * H; t += NW * 32) {
+            const int kz = t % H, gj = t / H, j2 = gj % N2, g = gj / N2;
+            const float2 *src = src0 + (size_t)g * (D * D * H) + j2 * H + kz;
+            float2 v[N1];
+#pragma unroll
+            for (int j1 = 0; j1 < N1; ++j1) v[j1] = src[N2 * j1 * H];
+            rdft_plan<N1, true, N2>(v, twn);
+            float2 *col = buf + g * CS + j2 * RS + kz;
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) col[N2 * k1 * RS] = (k1 && j2) ? twiddle<true>(v[k1], twn[j2 * k1]) : v[k1];
+        }
+        __syncthreads();
+        for (int t = threadIdx.x; t < NGRP * N1 * H; t += NW * 32) {
+            const int kz = t % H, gk = t / H, k1 = gk % N1, g = gk / N1;
+            float2 *col = buf + g * CS + N2 * k1 * RS + kz;
+            float2 u[N2];
+#pragma unroll
+            for (int j2 = 0; j2 < N2; ++j2) u[j2] = col[j2 * RS];
+            rdft_plan<N2, true, N1>(u, twn);
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2) col[k2 * RS] = u[k2];
+        }
+        __syncthreads();
+    } else {
+        // inverse y step 2 from U: items (g, k1, kz) -> rows N2 k1 + j2
+        for (int t = threadIdx.x; t < NGRP * N1 * H; t += NW * 32) {
+            const int kz = t % H, gk = t / H, k1 = gk % N1, g = gk / N1;
+            const float2 *src = src0 + (size_t)g * (D * D * H) + k1 * H + kz;
+            float2 u[N2];
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2) u[k2] = src[N1 * k2 * H];
+            rdft<N2, true>(u);
+            float2 *col = buf + g * CS + N2 * k1 * RS + kz;
+#pragma unroll
+            for (int j2 = 0; j2 < N2; ++j2) col[j2 * RS] = (k1 && j2) ? cmulc(u[j2], twn[j2 * k1]) : u[j2];
+        }
+        __syncthreads();
+        // inverse y step 1, in place: items (g, j2, kz) -> rows y = j2 + N2 j1
+        for (int t = threadIdx.x; t < NGRP * N2 * H; t += NW * 32) {
+            const int kz = t % H, gj = t / H, j2 = gj % N2, g = gj / N2;
+            float2 *col = buf + g * CS + j2 * RS + kz;
+            float2 v[N1];
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) v[k1] = col[N2 * k1 * RS];
+            rdft<N1, true>(v);
+#pragma unroll
+            for (int j1 = 0; j1 < N1; ++j1) col[N2 * j1 * RS] = v[j1];
+        }
+        __syncthreads();
+    }
+    const int p0 = warp * PL, pn = min(PL, NP - p0);   // pn <= 0: no line left for this warp
+    unsigned long long best[3] = {0ull, 0ull, 0ull};
+    // scores s0 (and s1) of voxel (y, z)
+    auto score = [&](float s0, float s1, int y, int z) {
+        const uint32_t lin = (uint32_t)((x * D + y) * D + z);
+        best[0] = max(best[0], make_key(s0, lin));
+        if (SC >= 2) best[1] = max(best[1], make_key(s1, lin));
+        if (SC == 3) {
+            const float sv = __fdiv_rn(__fsub_rn(s0, a.mix.vave), a.mix.vstd);
+            const float sp = __fdiv_rn(__fsub_rn(s1, a.mix.pave), a.mix.pstd);
+            best[2] = max(best[2], make_key(__fadd_rn(__fmul_rn(a.mix.one_minus_alpha, sv),
+                                                      __fmul_rn(a.mix.alpha, sp)), lin));
+        }
+    };
+    if constexpr (!PFA) {
+        // z in the forward's order, each line in its own two rows' storage (elements
+        // of k1 < KH in the first row's, the others in the second's): rows (2p, 2p + 1)
+        // as one full line (Hermitian completion, DC and Nyquist imaginary parts
+        // dropped); step 1: items (g, line, j2), whole lines per round, read before
+        // they are written; step 2 and scores: items (line, k1) over every group
+        constexpr int KH = (N1 + 1) / 2, LPR = 32 / N2;
+        auto row_at = [](int y) { return (N2 * (y % N1) + y / N1) * RS; };
+        const int lj2 = lane % N2, lq = lane / N2;
+#pragma unroll 1
+        for (int l0 = 0; l0 < NGRP * pn; l0 += LPR) {
+            const int l = l0 + lq, g = NGRP == 2 ? l / max(pn, 1) : 0, p = p0 + l - g * pn;
+            const bool on = lq < LPR && l < NGRP * pn;
+            const bool hb = 2 * p + 1 < D;
+            float2 *ra = buf + g * CS + row_at(2 * p), *rb = hb ? buf + g * CS + row_at(2 * p + 1) : buf + g * CS + D * RS;
+            float2 v[N1];
+            if (on) {
+#pragma unroll
+                for (int j1 = 0; j1 < N1; ++j1) {
+                    const int k = lj2 + N2 * j1;
+                    const bool low = k < H;
+                    const int kk = low ? k : D - k;
+                    float2 A = ra[kk], B = hb ? rb[kk] : make_float2(0.f, 0.f);
+                    if (k == 0 || 2 * k == D) { A.y = 0.f; B.y = 0.f; }
+                    v[j1] = low ? make_float2(A.x - B.y, A.y + B.x) : make_float2(A.x + B.y, B.x - A.y);
+                }
+                rdft_plan<N1, true, N2>(v, twn);
+            }
+            __syncwarp();
+            if (on)
+#pragma unroll
+                for (int k1 = 0; k1 < N1; ++k1)
+                    (k1 < KH ? ra + P2 * k1 : rb + P2 * (k1 - KH))[lj2] = (k1 && lj2) ? twiddle<true>(v[k1], twn[lj2 * k1]) : v[k1];
+        }
+        __syncwarp();
+        for (int t = lane; t < pn * N1; t += 32) {
+            const int k1 = t % N1, p = p0 + t / N1;
+            const bool hb = 2 * p + 1 < D;
+            const int at = k1 < KH ? row_at(2 * p) + P2 * k1 : (hb ? row_at(2 * p + 1) : D * RS) + P2 * (k1 - KH);
+            float2 u0[N2], u1[N2];
+#pragma unroll
+            for (int j2 = 0; j2 < N2; ++j2) u0[j2] = buf[at + j2];
+            rdft_plan<N2, true, N1>(u0, twn);
+            if (NGRP == 2) {
+#pragma unroll
+                for (int j2 = 0; j2 < N2; ++j2) u1[j2] = buf[CS + at + j2];
+                rdft_plan<N2, true, N1>(u1, twn);
+            }
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2) {
+                const int z = k1 + N1 * k2;
+                score(u0[k2].x, NGRP == 2 ? u1[k2].x : 0.f, 2 * p, z);
+                if (hb) score(u0[k2].y, NGRP == 2 ? u1[k2].y : 0.f, 2 * p + 1, z);
+            }
+        }
+    } else {
+        // z: rows (2p, 2p + 1) as one full line (Hermitian completion, DC and Nyquist
+        // imaginary parts dropped), inverse step 2 in the rows' own storage: items
+        // (g, line, k1), whole lines per round, read before they are written
+        constexpr int LPR = 32 / N1;
+        const int lk1 = lane % N1, lq = lane / N1;
+#pragma unroll 1
+        for (int l0 = 0; l0 < NGRP * pn; l0 += LPR) {
+            const int l = l0 + lq, g = NGRP == 2 ? l / max(pn, 1) : 0, p = p0 + l - g * pn;
+            const bool on = lq < LPR && l < NGRP * pn;
+            float2 *line = buf + g * CS + p * LS;
+            const bool hb = 2 * p + 1 < D;
+            float2 u[N2];
+            if (on) {
+#pragma unroll
+                for (int k2 = 0; k2 < N2; ++k2) {
+                    const int k = lk1 + N1 * k2;
+                    if (k < H) {
+                        float2 A = line[k], B = hb ? line[RS + k] : make_float2(0.f, 0.f);
+                        if (k == 0 || 2 * k == D) { A.y = 0.f; B.y = 0.f; }
+                        u[k2] = make_float2(A.x - B.y, A.y + B.x);
+                    } else {
+                        const float2 A = line[D - k], B = hb ? line[RS + D - k] : make_float2(0.f, 0.f);
+                        u[k2] = make_float2(A.x + B.y, B.x - A.y);
+                    }
+                }
+                rdft<N2, true>(u);
+            }
+            __syncwarp();
+            if (on)
+#pragma unroll
+                for (int j2 = 0; j2 < N2; ++j2)
+                    line[P2 * lk1 + j2] = (lk1 && j2) ? cmulc(u[j2], twn[j2 * lk1]) : u[j2];
+        }
+        __syncwarp();
+        // inverse z step 1 and scores: items (line, j2) over every group
+        for (int t = lane; t < pn * N2; t += 32) {
+            const int j2 = t / pn, p = p0 + t - j2 * pn;
+            float2 v0[N1], v1[N1];
+            const float2 *l0 = buf + p * LS + j2;
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) v0[k1] = l0[P2 * k1];
+            rdft<N1, true>(v0);
+            if (NGRP == 2) {
+#pragma unroll
+                for (int k1 = 0; k1 < N1; ++k1) v1[k1] = l0[CS + P2 * k1];
+                rdft<N1, true>(v1);
+            }
+#pragma unroll
+            for (int j1 = 0; j1 < N1; ++j1) {
+                const int z = j2 + N2 * j1;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int y = 2 * p + half;
+                    if (y >= D) break;
+                    score(half ? v0[j1].y : v0[j1].x, NGRP == 2 ? (half ? v1[j1].y : v1[j1].x) : 0.f, y, z);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < SC; ++s) {
+        const unsigned long long v = warp_max_u64(best[s]);
+        if (lane == 0) red[s * 8 + warp] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < SC) {
+        unsigned long long v = 0ull;
+        for (int w = 0; w < NW; ++w) v = max(v, red[threadIdx.x * 8 + w]);
+        atomicMax(&a.keys[(size_t)r * a.nscore + threadIdx.x], v);
+    }
+}
+
+}  // namespace vg
