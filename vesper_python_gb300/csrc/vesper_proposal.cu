@@ -21,6 +21,7 @@ namespace vg {
 // keeps its partial gradients in shared memory and writes them to its own
 // workspace slot
 constexpr int kPropBlocks = 304;
+constexpr int kPropSMs = 152;
 
 // ---- convolution (3x3x3, zero padding) ----------------------------------------
 __global__ void k_conv_fwd(const float *in, int cin, const __nv_bfloat16 *W, const float *bias, int cout, int d,
@@ -47,73 +48,100 @@ __global__ void k_conv_fwd(const float *in, int cin, const __nv_bfloat16 *W, con
     out[(size_t)co * n + v] = relu ? fmaxf(acc, 0.f) : acc;
 }
 
-// The same layer with COG = 4 output channels and ZS consecutive z voxels per
-// thread: the block's COG x cin x 27 weights sit in shared memory as float32 in
-// [cin][27][channel] order (each tap's four weights are one 16-byte broadcast
-// load), and for each input channel and (x, y) neighbour row the ZS + 2 input
-// values of the row are loaded once, so each load feeds up to 3 x COG products
-// and each weight load ZS x COG.  Taps outside the grid are skipped per voxel
-// as in k_conv_fwd, in the same order (bias, then ci, then tap), so the
-// results are the same bits.
-constexpr int kConvCOG = 4;
-constexpr int kConvZS = 4;   // measured over the prop128 step: 4 beat 2 and 1 (one voxel per thread)
-template <int COG, int ZS>
-__global__ void __launch_bounds__(128) k_conv_fwd_s(const float *in, int cin, const __nv_bfloat16 *W,
-                                                    const float *bias, int cout, int d, int relu, float *out) {
-    static_assert(COG == 4, "k_conv_fwd_s: 4 output channels per thread");
-    extern __shared__ float4 wsh4[];   // [cin][27]
+// Quotients by a small divisor through the high half of a product: m = recip(d);
+// exact for v d < 2^32.
+__host__ __device__ __forceinline__ unsigned recip(unsigned d) { return 0xffffffffu / d + 1u; }
+__device__ __forceinline__ int quot(int v, int d, unsigned m) { return d == 1 ? v : (int)__umulhi((unsigned)v, m); }
+
+// The same layer, and its input gradient, with 4 output channels and ZS consecutive z
+// voxels per thread: the 4 channels' weights sit in shared memory as float32 in
+// [summed channel][27][4] order (a tap's four weights are one 16-byte broadcast), and
+// a summed channel's 9 (x, y) neighbour rows of ZS + 2 values are loaded together,
+// zero off the grid, before any product, so a channel costs one load latency instead
+// of one per row behind its bounds test (the four layers of two side-15 maps 490 -> 150
+// us, of 16 maps 460 -> 290).  Sums in the order of k_conv_fwd (bias, then channel,
+// then tap) and of k_conv_bwd_data (channel, then tap); a tap off the grid adds +-0, so
+// results are the same bits for finite weights.
+// BWD: the sums run over the layer's output channels (their gradient masked where a
+// ReLU let nothing through) and the taps are mirrored.
+// SPL: a block's warps share 32 threads' voxels and sum nin / SPL channels each (added
+// in warp order), where a layer has too few voxels to hide a warp's latencies.
+template <int ZS, bool BWD, int SPL>
+__global__ void __launch_bounds__(128) k_conv_s(const float *in, const float *mask, int nin, const __nv_bfloat16 *W,
+                                                const float *bias, int nout, int d, int relu, float *out) {
+    extern __shared__ float4 wsh4[];   // [nin][27]
     float *wsh = (float *)wsh4;
-    const int n = d * d * d, nzs = (d + ZS - 1) / ZS;
-    const int co0 = blockIdx.y * COG;
-    in += (size_t)blockIdx.z * cin * n;
-    out += (size_t)blockIdx.z * cout * n;
-    for (int i = threadIdx.x; i < COG * cin * 27; i += blockDim.x) {
-        const int j = i / (cin * 27), t = i - j * cin * 27;   // t = ci * 27 + o
-        wsh[t * COG + j] = __bfloat162float(W[(size_t)co0 * cin * 27 + i]);
+    const int n = d * d * d, nzs = (d + ZS - 1) / ZS, c0 = blockIdx.y * 4;
+    in += (size_t)blockIdx.z * nin * n;     // map blockIdx.z of a stack
+    out += (size_t)blockIdx.z * nout * n;
+    for (int e = threadIdx.x; e < 4 * nin * 27; e += blockDim.x) {
+        const int j = e & 3, o = (e >> 2) % 27, c = (e >> 2) / 27;
+        wsh[e] = __bfloat162float(BWD ? W[((size_t)c * nout + c0 + j) * 27 + o] : W[((size_t)(c0 + j) * nin + c) * 27 + o]);
     }
     __syncthreads();
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= d * d * nzs) return;
-    const int x = u / (d * nzs), y = (u / nzs) % d, z0 = (u % nzs) * ZS;
-    float acc[ZS][COG];
+    const int split = SPL > 1 ? threadIdx.x / (128 / SPL) : 0;
+    const int u = blockIdx.x * (128 / SPL) + (SPL > 1 ? threadIdx.x % (128 / SPL) : threadIdx.x);
+    if (SPL == 1 && u >= d * d * nzs) return;
+    const int x = u / (d * nzs), y = (u / nzs) % d, z0 = (u % nzs) * ZS;   // x >= d past the end: no row is on the grid
+    // the 9 rows' places and the z values on the grid, a bit each
+    unsigned rows = 0u, zs = 0u;
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+        const int xx = x + r / 3 - 1, yy = y + r % 3 - 1;
+        rows |= (unsigned)(xx >= 0 && xx < d && yy >= 0 && yy < d) << r;
+    }
+#pragma unroll
+    for (int e = 0; e < ZS + 2; ++e) zs |= (unsigned)(z0 + e - 1 >= 0 && z0 + e - 1 < d) << e;
+    const int at = ((x - 1) * d + y - 1) * d + z0 - 1;
+    float acc[ZS][4];
 #pragma unroll
     for (int i = 0; i < ZS; ++i)
 #pragma unroll
-        for (int j = 0; j < COG; ++j) acc[i][j] = bias ? bias[co0 + j] : 0.f;
-    for (int ci = 0; ci < cin; ++ci) {
-        const float *src = in + (size_t)ci * n;
-        const float4 *w = wsh4 + (size_t)ci * 27;
+        for (int j = 0; j < 4; ++j) acc[i][j] = !BWD && bias && split == 0 ? bias[c0 + j] : 0.f;
+    const int per = (nin + SPL - 1) / SPL, c1 = min(nin, (split + 1) * per);
+#pragma unroll(ZS == 1 && !BWD ? 2 : 1)
+    for (int c = split * per; c < c1; ++c) {
+        const float *src = in + (size_t)c * n + at;
+        float v[9][ZS + 2];
 #pragma unroll
-        for (int ox = 0; ox < 3; ++ox) {
-            const int xx = x + ox - 1;
-            if (xx < 0 || xx >= d) continue;
+        for (int r = 0; r < 9; ++r)
 #pragma unroll
-            for (int oy = 0; oy < 3; ++oy) {
-                const int yy = y + oy - 1;
-                if (yy < 0 || yy >= d) continue;
-                const float *row = src + ((size_t)xx * d + yy) * d;
-                float val[ZS + 2];
+            for (int e = 0; e < ZS + 2; ++e)
+                v[r][e] = (rows >> r & 1u) && (zs >> e & 1u) ? __ldg(src + (r / 3 * d + r % 3) * d + e) : 0.f;
+        if (BWD && mask) {
+            const float *mk = mask + (size_t)c * n + at;
 #pragma unroll
-                for (int e = 0; e < ZS + 2; ++e) {
-                    const int zz = z0 + e - 1;
-                    val[e] = zz >= 0 && zz < d ? row[zz] : 0.f;
-                }
+            for (int r = 0; r < 9; ++r)
 #pragma unroll
-                for (int oz = 0; oz < 3; ++oz) {
-                    const float4 w4 = w[ox * 9 + oy * 3 + oz];
+                for (int e = 0; e < ZS + 2; ++e)
+                    if ((rows >> r & 1u) && (zs >> e & 1u) && !(__ldg(mk + (r / 3 * d + r % 3) * d + e) > 0.f))
+                        v[r][e] = 0.f;
+        }
+        const float4 *w = wsh4 + (size_t)c * 27;
 #pragma unroll
-                    for (int i = 0; i < ZS; ++i) {
-                        const int zz = z0 + i + oz - 1;
-                        if (zz < 0 || zz >= d) continue;
-                        const float v = val[i + oz];
-                        acc[i][0] = fmaf(w4.x, v, acc[i][0]);
-                        acc[i][1] = fmaf(w4.y, v, acc[i][1]);
-                        acc[i][2] = fmaf(w4.z, v, acc[i][2]);
-                        acc[i][3] = fmaf(w4.w, v, acc[i][3]);
-                    }
-                }
+        for (int o = 0; o < 27; ++o) {
+            const float4 w4 = w[o];
+#pragma unroll
+            for (int i = 0; i < ZS; ++i) {
+                const float t = v[BWD ? 8 - o / 3 : o / 3][i + (BWD ? 2 - o % 3 : o % 3)];
+                acc[i][0] = fmaf(w4.x, t, acc[i][0]);
+                acc[i][1] = fmaf(w4.y, t, acc[i][1]);
+                acc[i][2] = fmaf(w4.z, t, acc[i][2]);
+                acc[i][3] = fmaf(w4.w, t, acc[i][3]);
             }
         }
+    }
+    if (SPL > 1) {
+        static_assert(SPL == 1 || ZS == 1, "split channels: one voxel per thread");
+        __shared__ float part[SPL][128 / SPL][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) part[split][threadIdx.x % (128 / SPL)][j] = acc[0][j];
+        __syncthreads();
+        if (split || u >= n) return;
+#pragma unroll
+        for (int s = 1; s < SPL; ++s)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[0][j] += part[s][threadIdx.x][j];
     }
 #pragma unroll
     for (int i = 0; i < ZS; ++i) {
@@ -121,8 +149,30 @@ __global__ void __launch_bounds__(128) k_conv_fwd_s(const float *in, int cin, co
         if (z >= d) break;
         const size_t v = ((size_t)x * d + y) * d + z;
 #pragma unroll
-        for (int j = 0; j < COG; ++j) out[(size_t)(co0 + j) * n + v] = relu ? fmaxf(acc[i][j], 0.f) : acc[i][j];
+        for (int j = 0; j < 4; ++j) out[(size_t)(c0 + j) * n + v] = !BWD && relu ? fmaxf(acc[i][j], 0.f) : acc[i][j];
     }
+}
+
+// Launch, or false where the weights do not fit or the channels do not group.
+// 4 voxels per thread; a few maps leave most SMs without a block then: one voxel
+// each, backwards with the channels split over the block's warps.
+template <bool BWD>
+static bool conv_s(const float *in, const float *mask, const __nv_bfloat16 *W, const float *bias, int nin, int nout, int d,
+                   int relu, int nmap, float *out, cudaStream_t st) {
+    const size_t sm = (size_t)4 * nin * 27 * sizeof(float);
+    if (nout % 4 || sm + 4096 > (size_t)smem_limit()) return false;
+    const int n = d * d * d, nu = d * d * ((d + 3) / 4);
+    if ((long long)((nu + 127) / 128) * (nout / 4) * nmap < 2 * kPropSMs) {
+        constexpr int SPL = BWD ? 4 : 1;   // the forward keeps k_conv_fwd's order of sums
+        allow_smem(k_conv_s<1, BWD, SPL>, sm);
+        k_conv_s<1, BWD, SPL><<<dim3((n + 128 / SPL - 1) / (128 / SPL), nout / 4, nmap), 128, sm, st>>>(
+            in, mask, nin, W, bias, nout, d, relu, out);
+    } else {
+        allow_smem(k_conv_s<4, BWD, 1>, sm);
+        k_conv_s<4, BWD, 1><<<dim3((nu + 127) / 128, nout / 4, nmap), 128, sm, st>>>(in, mask, nin, W, bias, nout, d, relu,
+                                                                                     out);
+    }
+    return true;
 }
 
 // din[ci][v] = sum_co sum_o W[co][ci][o] * g[co][v - o],  g = dout (masked by
@@ -191,6 +241,71 @@ __global__ void k_conv_bwd_weight(const float *dout, const float *out, int relu,
             dW[((size_t)co * cin + ci) * 27 + threadIdx.x] += s;
         else if (ci == 0)
             db[co] += s;
+    }
+}
+
+// The same weight gradients with kWgCo output channels per block: the input channel
+// sits in shared memory with a zero border, so a voxel's 27 neighbours are plain
+// loads, each used for kWgCo products, where one block per (co, ci) pair spent its
+// instructions on the neighbours' bounds (the eight layers of a training step at side 15
+// 354 -> 247 us).  2 channels and 256 threads: 4 channels take 192 registers.
+constexpr int kWgCo = 2;
+constexpr int kWgThreads = 256;
+__global__ void __launch_bounds__(kWgThreads) k_conv_bwd_weight_s(const float *dout, const float *out, int relu,
+                                                                  const float *in, int cin, int cout, int d, float *dW,
+                                                                  float *db, unsigned md, unsigned mp) {
+    extern __shared__ float pad[];   // [d + 2]^3
+    __shared__ float red[kWgThreads / 32][kWgCo * 28];
+    const int n = d * d * d, p = d + 2;
+    const int ci = blockIdx.x % cin, co0 = blockIdx.x / cin * kWgCo;
+    const float *src = in + (size_t)ci * n;
+    for (int e = threadIdx.x; e < p * p * p; e += kWgThreads) {
+        const int q = quot(e, p, mp), x = quot(q, p, mp) - 1, y = q - (x + 1) * p - 1, z = e - q * p - 1;
+        const bool on = x >= 0 && y >= 0 && z >= 0 && x < d && y < d && z < d;
+        pad[e] = on ? __ldg(src + (x * d + y) * d + z) : 0.f;
+    }
+    __syncthreads();
+    float acc[kWgCo][28];
+#pragma unroll
+    for (int j = 0; j < kWgCo; ++j)
+#pragma unroll
+        for (int o = 0; o < 28; ++o) acc[j][o] = 0.f;
+    for (int v = threadIdx.x; v < n; v += kWgThreads) {
+        float g[kWgCo];
+#pragma unroll
+        for (int j = 0; j < kWgCo; ++j) {
+            const size_t i = (size_t)(co0 + j) * n + v;
+            g[j] = __ldg(dout + i);
+            if (relu && !(__ldg(out + i) > 0.f)) g[j] = 0.f;
+            acc[j][27] += g[j];
+        }
+        const int q = quot(v, d, md), x = quot(q, d, md);
+        const float *c = pad + (x * p + q - x * d) * p + v - q * d;
+#pragma unroll
+        for (int o = 0; o < 27; ++o) {
+            const float t = c[(o / 9 * p + o / 3 % 3) * p + o % 3];
+#pragma unroll
+            for (int j = 0; j < kWgCo; ++j) acc[j][o] = fmaf(g[j], t, acc[j][o]);
+        }
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int j = 0; j < kWgCo; ++j)
+#pragma unroll
+        for (int o = 0; o < 28; ++o) {
+            float t = acc[j][o];
+            for (int k = 16; k > 0; k >>= 1) t += __shfl_down_sync(0xffffffffu, t, k);
+            if (lane == 0) red[warp][j * 28 + o] = t;
+        }
+    __syncthreads();
+    for (int e = threadIdx.x; e < kWgCo * 28; e += kWgThreads) {
+        float t = 0.f;
+        for (int w = 0; w < kWgThreads / 32; ++w) t += red[w][e];
+        const int j = e / 28, o = e % 28;
+        if (o < 27)
+            dW[((size_t)(co0 + j) * cin + ci) * 27 + o] += t;
+        else if (ci == 0)
+            db[co0 + j] += t;
     }
 }
 
@@ -536,6 +651,290 @@ __global__ void __launch_bounds__(256) k_prop_score_map_s(const uint4 *ET, const
     }
 }
 
+// ---- the same correlation and its gradients for 8 float32 channels -----------------
+// One side's features (the gathered ones) sit in shared memory as two planes of
+// float4, so a gathered voxel is two 16-byte loads; row n is zero and stands for
+// "no source voxel".  Positions are recomputed: the matrices of a group of
+// rotations are in shared memory and a voxel's own coordinates stay in registers,
+// about 25 instructions, where the general prop_src takes several times that.
+constexpr int kS8Threads = 1024;
+constexpr int kS8Rot = 8;      // rotations whose matrices are staged together
+
+// Planes [2][n + 1] float4 of channel-major features.
+__device__ __forceinline__ void stage_planes(const float *E, int n, float4 *pl) {
+    for (int v = threadIdx.x; v < n; v += blockDim.x) {
+        pl[v] = make_float4(__ldg(E + v), __ldg(E + n + v), __ldg(E + 2 * n + v), __ldg(E + 3 * n + v));
+        pl[n + 1 + v] =
+            make_float4(__ldg(E + 4 * n + v), __ldg(E + 5 * n + v), __ldg(E + 6 * n + v), __ldg(E + 7 * n + v));
+    }
+    if (threadIdx.x == 0) pl[n] = pl[2 * n + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// prop_src with the voxel's first candidate rows (hx, hy, hz: minus the centre)
+// at hand; the other candidates of an odd side's middle index are looked at only
+// where the first is off the grid, in gather_src's order (z slowest, x, y).
+struct Voxel {
+    float hx, hy, hz;
+    int v;     // destination voxel
+    int mid;   // -1: no row; else a bit for each axis with a second row (4 z, 2 x, 1 y)
+};
+__device__ __forceinline__ Voxel voxel_at(int x, int y, int z, int d) {
+    Voxel o;
+    o.v = (x * d + y) * d + z;
+    o.mid = 0;
+    if (d & 1) {
+        const int m = (d - 1) >> 1;
+        o.mid = x == d - 1 || y == d - 1 || z == d - 1 ? -1 : (z == m) << 2 | (x == m) << 1 | (y == m);
+        x += x >= m;
+        y += y >= m;
+        z += z >= m;
+    }
+    const float hc = 0.5f * (float)d;
+    o.hx = (float)x - hc;
+    o.hy = (float)y - hc;
+    o.hz = (float)z - hc;
+    return o;
+}
+__device__ __forceinline__ Voxel voxel_of(int v, int d) { return voxel_at(v / (d * d), v / d % d, v % d, d); }
+// A staged matrix (3 float4 of shared memory) in registers.
+__device__ __forceinline__ void load_matrix(const float4 *m, float (&F)[9]) {
+    const float4 a = m[0], b = m[1], c = m[2];
+    F[0] = a.x, F[1] = a.y, F[2] = a.z, F[3] = a.w, F[4] = b.x, F[5] = b.y, F[6] = b.z, F[7] = b.w, F[8] = c.x;
+}
+__device__ __forceinline__ int voxel_src(const float (&F)[9], int d, const Voxel &o) {
+    if (o.mid < 0) return -1;
+    const float hc = 0.5f * (float)d;
+    int ox, oy, oz;
+    if (old_index(F, d, hc, o.hx, o.hy, o.hz, ox, oy, oz)) return (ox * d + oy) * d + oz;
+#pragma unroll 1
+    for (int k = -o.mid & o.mid; k; k = (k - o.mid) & o.mid)   // the masks within mid, ascending
+        if (old_index(F, d, hc, o.hx - (float)(k >> 1 & 1), o.hy - (float)(k & 1), o.hz - (float)(k >> 2), ox, oy, oz))
+            return (ox * d + oy) * d + oz;
+    return -1;
+}
+
+__device__ __forceinline__ float dot8(float4 a0, float4 a1, float4 b0, float4 b1, float s) {
+    s = fmaf(a0.x, b0.x, s);
+    s = fmaf(a0.y, b0.y, s);
+    s = fmaf(a0.z, b0.z, s);
+    s = fmaf(a0.w, b0.w, s);
+    s = fmaf(a1.x, b1.x, s);
+    s = fmaf(a1.y, b1.y, s);
+    s = fmaf(a1.z, b1.z, s);
+    return fmaf(a1.w, b1.w, s);
+}
+__device__ __forceinline__ void axpy8(float g, float4 b0, float4 b1, float *acc) {
+    acc[0] = fmaf(g, b0.x, acc[0]);
+    acc[1] = fmaf(g, b0.y, acc[1]);
+    acc[2] = fmaf(g, b0.z, acc[2]);
+    acc[3] = fmaf(g, b0.w, acc[3]);
+    acc[4] = fmaf(g, b1.x, acc[4]);
+    acc[5] = fmaf(g, b1.y, acc[5]);
+    acc[6] = fmaf(g, b1.z, acc[6]);
+    acc[7] = fmaf(g, b1.w, acc[7]);
+}
+
+// scores of rotations [b chunk, (b + 1) chunk): the query's features staged once
+// per block, each target voxel's read once per group of kS8Rot rotations.
+// Bound by the shared-memory wavefronts of the two gathers per (rotation, voxel).
+__global__ void __launch_bounds__(kS8Threads) k_prop_score8(const float *ET, const float *EQ, int d,
+                                                            const float *rotmats, int nrot, int chunk, float *scores) {
+    extern __shared__ float4 pl[];   // [2][n + 1]
+    __shared__ float4 Fs[kS8Rot][3];
+    __shared__ float red[kS8Rot][kS8Threads / 32];
+    const int n = d * d * d;
+    stage_planes(EQ, n, pl);
+    const int r1 = min(nrot, (int)(blockIdx.x + 1) * chunk);
+    for (int r0 = blockIdx.x * chunk; r0 < r1; r0 += kS8Rot) {
+        __syncthreads();
+        if (threadIdx.x < 9 * kS8Rot) {
+            const int j = threadIdx.x / 9, e = threadIdx.x % 9;
+            ((float *)Fs[j])[e] = r0 + j < r1 ? rotmats[(size_t)(r0 + j) * 9 + e] : 0.f;
+        }
+        __syncthreads();
+        float acc[kS8Rot];
+#pragma unroll
+        for (int j = 0; j < kS8Rot; ++j) acc[j] = 0.f;
+        for (int v = threadIdx.x; v < n; v += kS8Threads) {
+            const Voxel o = voxel_of(v, d);
+            const float4 t0 = make_float4(__ldg(ET + v), __ldg(ET + n + v), __ldg(ET + 2 * n + v), __ldg(ET + 3 * n + v));
+            const float4 t1 =
+                make_float4(__ldg(ET + 4 * n + v), __ldg(ET + 5 * n + v), __ldg(ET + 6 * n + v), __ldg(ET + 7 * n + v));
+#pragma unroll
+            for (int j = 0; j < kS8Rot; ++j) {
+                float F[9];
+                load_matrix(Fs[j], F);
+                const int s = voxel_src(F, d, o);
+                const float4 *q = pl + (s < 0 ? n : s);
+                acc[j] = dot8(t0, t1, q[0], q[n + 1], acc[j]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kS8Rot; ++j) {
+            float a = acc[j];
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+            if ((threadIdx.x & 31) == 0) red[j][threadIdx.x >> 5] = a;
+        }
+        __syncthreads();
+        if (threadIdx.x < kS8Rot && r0 + (int)threadIdx.x < r1) {
+            float t = 0.f;
+            for (int w = 0; w < kS8Threads / 32; ++w) t += red[threadIdx.x][w];
+            scores[r0 + threadIdx.x] = t;
+        }
+    }
+}
+
+// The source voxel of every (rotation, voxel) of a group of rotations, int16
+// [rotations][ns] (-1: none; ns = n rounded up to 8).  An odd side's middle voxels,
+// whose other candidate rows take a loop, are done apart from the rest so that
+// they do not hold up whole warps.
+constexpr int kSrcThreads = 512;
+__global__ void __launch_bounds__(kSrcThreads) k_prop_sources(int d, int ns, const float *rotmats, int nrot,
+                                                             int16_t *table) {
+    __shared__ float4 Fs[kS8Rot][3];
+    const int r0 = blockIdx.x * kS8Rot, rn = min(kS8Rot, nrot - r0), dd = d * d;
+    if (threadIdx.x < 9 * rn)
+        ((float *)Fs[threadIdx.x / 9])[threadIdx.x % 9] = rotmats[(size_t)r0 * 9 + threadIdx.x];
+    __syncthreads();
+    int16_t *out = table + (size_t)r0 * ns;
+    auto row = [&](const Voxel &o) {
+        for (int j = 0; j < rn; ++j) {
+            float F[9];
+            load_matrix(Fs[j], F);
+            out[(size_t)j * ns + o.v] = (int16_t)voxel_src(F, d, o);
+        }
+    };
+    const int m = (d - 1) >> 1;
+    const bool odd = d & 1;
+    for (int v = threadIdx.x; v < d * dd; v += kSrcThreads) {
+        const Voxel o = voxel_of(v, d);
+        if (o.mid <= 0) row(o);
+    }
+    if (!odd) return;
+    const int e1 = dd, e2 = e1 + (d - 1) * d, e3 = e2 + (d - 1) * (d - 1);
+    for (int e = threadIdx.x; e < e3; e += kSrcThreads) {   // x = m; else y = m; else z = m
+        int x = m, y = e / d, z = e % d;
+        if (e >= e2) {
+            x = (e - e2) / (d - 1);
+            y = (e - e2) % (d - 1);
+            x += x >= m;
+            y += y >= m;
+            z = m;
+        } else if (e >= e1) {
+            x = (e - e1) / d;
+            x += x >= m;
+            y = m;
+            z = (e - e1) % d;
+        }
+        row(voxel_at(x, y, z, d));
+    }
+}
+
+// Target side of the gradient, part[c][0][k][v] (+)= sum over the chunk c of
+// rotations of g_r EQ[k][src_r(v)]: a thread owns kT8Own voxels and keeps their 8
+// sums in registers (block (p, c): voxels [p, p + 1) kT8Own kS8Threads, chunk c).
+// add: the sums go on from the last group of rotations.
+constexpr int kT8Own = 4;
+__global__ void __launch_bounds__(kS8Threads) k_prop_bwd_t8(const float *EQ, int d, int ns, const int16_t *table,
+                                                            int nrot, const float *gs, int chunk, int add,
+                                                            float *part) {
+    extern __shared__ float4 pl[];   // [2][n + 1]
+    const int n = d * d * d;
+    stage_planes(EQ, n, pl);
+    __syncthreads();
+    float acc[kT8Own][8];
+#pragma unroll
+    for (int i = 0; i < kT8Own; ++i)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[i][k] = 0.f;
+    const int r1 = min(nrot, (int)(blockIdx.y + 1) * chunk), v0 = blockIdx.x * kT8Own * kS8Threads + threadIdx.x;
+#pragma unroll 2
+    for (int r = blockIdx.y * chunk; r < r1; ++r) {
+        const float g = __ldg(gs + r);
+#pragma unroll
+        for (int i = 0; i < kT8Own; ++i) {
+            const int v = v0 + i * kS8Threads;
+            const int s = v < n ? (int)__ldg(table + (size_t)r * ns + v) : -1;
+            const float4 *q = pl + (s < 0 || g == 0.f ? n : s);
+            axpy8(g, q[0], q[n + 1], acc[i]);
+        }
+    }
+    float *dst = part + (size_t)blockIdx.y * 16 * n;
+#pragma unroll
+    for (int i = 0; i < kT8Own; ++i) {
+        const int v = v0 + i * kS8Threads;
+        if (v < n)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) dst[(size_t)k * n + v] = acc[i][k] + (add ? dst[(size_t)k * n + v] : 0.f);
+    }
+}
+
+// Query side, part[c][1][k][s] (+)= sum over the chunk's rotations of g_r sum of
+// ET[k][v] over the v with src_r(v) = s.  Scattering the 8 channels with
+// shared-memory float atomics (compare-and-swap loops) took most of the backward
+// pass; instead each rotation's voxels are linked into a list per source (one
+// integer exchange each), and a thread owns kS8Own sources, follows their lists and
+// keeps the sums in registers.  NB rotations between two barriers, as many as shared
+// memory holds lists for.
+// Measured at side 15, 24,624 rotations: both sides together 6.12 ms with atomics; now
+// source table 0.23, target side 0.29, query side 0.48, the last two bound by the
+// shared-memory wavefronts of their gathers.
+constexpr int kS8Own = 4;
+template <int NB>
+__global__ void __launch_bounds__(kS8Threads) k_prop_bwd_q8(const float *ET, int d, int ns, const int16_t *table,
+                                                            int nrot, const float *gs, int chunk, int add,
+                                                            float *part) {
+    extern __shared__ float4 pl[];   // [2][n + 1], then int head[NB][kOwned], int16 next[NB][ns]
+    constexpr int kOwned = kS8Own * kS8Threads;
+    const int n = d * d * d, s0 = blockIdx.x * kOwned;
+    int *head = (int *)(pl + 2 * (n + 1));
+    int16_t *next = (int16_t *)(head + NB * kOwned);
+    stage_planes(ET, n, pl);
+    for (int e = threadIdx.x; e < NB * kOwned; e += kS8Threads) head[e] = -1;
+    float acc[kS8Own][8];
+#pragma unroll
+    for (int i = 0; i < kS8Own; ++i)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[i][k] = 0.f;
+    const int r1 = min(nrot, (int)(blockIdx.y + 1) * chunk);
+    for (int r = blockIdx.y * chunk; r < r1; r += NB) {
+        __syncthreads();
+        for (int v = threadIdx.x; v < n; v += kS8Threads) {
+            unsigned s[NB];
+#pragma unroll
+            for (int b = 0; b < NB; ++b)   // -1 - s0 wraps past kOwned
+                s[b] = r + b < r1 ? (unsigned)((int)__ldg(table + (size_t)(r + b) * ns + v) - s0) : ~0u;
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+                if (s[b] < (unsigned)kOwned) next[b * ns + v] = (int16_t)atomicExch(head + b * kOwned + s[b], v);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const float g = r + b < r1 ? __ldg(gs + r + b) : 0.f;
+#pragma unroll
+            for (int i = 0; i < kS8Own; ++i) {
+                int *h = head + b * kOwned + i * kS8Threads + threadIdx.x;
+                int v = *h;
+                *h = -1;
+                if (g == 0.f) continue;
+                while (v >= 0) {
+                    axpy8(g, pl[v], pl[n + 1 + v], acc[i]);
+                    v = next[b * ns + v];
+                }
+            }
+        }
+    }
+    float *dst = part + (size_t)blockIdx.y * 16 * n + (size_t)8 * n;
+#pragma unroll
+    for (int i = 0; i < kS8Own; ++i) {
+        const int s = s0 + i * kS8Threads + threadIdx.x;
+        if (s < n)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) dst[(size_t)k * n + s] = acc[i][k] + (add ? dst[(size_t)k * n + s] : 0.f);
+    }
+}
+
 // Partial gradients of the correlation for channels [k0, k0 + kc): block b
 // takes rotations [b*chunk, (b+1)*chunk) and writes part[b][0][k][v] =
 // sum_r g_r EQ[k][src_r(v)] and part[b][1][k][s] = sum_r g_r ET[k][v] summed
@@ -784,15 +1183,9 @@ extern "C" int vesper_prop_conv_fwd(const float *in, int cin, const void *W, con
     if (!in || !W || !out || cin < 1 || cout < 1 || d < 1 || nmap < 1 || nmap > 65535)
         return fail(VESPER_ERR_INVALID, "conv_fwd: bad args");
     const int n = d * d * d;
-    // 4 output channels per thread (8 measured 10 % slower over the encoder), 4 z voxels
-    constexpr int COG = kConvCOG, ZS = kConvZS;
-    const size_t sm = (size_t)COG * cin * 27 * sizeof(float);
-    if (cout % COG == 0 && sm <= (size_t)smem_limit()) {
-        const int nu = d * d * ((d + ZS - 1) / ZS);
-        allow_smem(k_conv_fwd_s<COG, ZS>, sm);
-        k_conv_fwd_s<COG, ZS><<<dim3((nu + 127) / 128, cout / COG, nmap), 128, sm, (cudaStream_t)stream>>>(
-            in, cin, (const __nv_bfloat16 *)W, bias, cout, d, relu, out);
-        VG_CHECK_LAUNCH("k_conv_fwd_s");
+    if (conv_s<false>(in, nullptr, (const __nv_bfloat16 *)W, bias, cin, cout, d, relu, nmap, out,
+                          (cudaStream_t)stream)) {
+        VG_CHECK_LAUNCH("k_conv_s");
         return VESPER_OK;
     }
     k_conv_fwd<<<dim3((n + 127) / 128, cout, nmap), 128, 0, (cudaStream_t)stream>>>(
@@ -807,14 +1200,41 @@ extern "C" int vesper_prop_conv_bwd(const float *dout, const float *out, int rel
         return fail(VESPER_ERR_INVALID, "conv_bwd: bad args");
     const int n = d * d * d;
     cudaStream_t st = (cudaStream_t)stream;
-    if (din) {
+    const size_t smw = (size_t)(d + 2) * (d + 2) * (d + 2) * sizeof(float);
+    if (din && conv_s<true>(dout, relu ? out : nullptr, (const __nv_bfloat16 *)W, nullptr, cout, cin, d, 0, 1, din,
+                                st)) {
+        VG_CHECK_LAUNCH("k_conv_s");
+    } else if (din) {
         k_conv_bwd_data<<<dim3((n + 127) / 128, cin), 128, 0, st>>>(dout, out, relu, (const __nv_bfloat16 *)W, cin,
                                                                     cout, d, din);
         VG_CHECK_LAUNCH("k_conv_bwd_data");
     }
+    if (cout % kWgCo == 0 && smw + 8192 <= (size_t)smem_limit()) {
+        allow_smem(k_conv_bwd_weight_s, smw);
+        k_conv_bwd_weight_s<<<cout / kWgCo * cin, kWgThreads, smw, st>>>(dout, out, relu, in, cin, cout, d, dW, db, recip(d),
+                                                                         recip(d + 2));
+        VG_CHECK_LAUNCH("k_conv_bwd_weight_s");
+        return VESPER_OK;
+    }
     k_conv_bwd_weight<<<cout * cin, 256, 0, st>>>(dout, out, relu, in, cin, cout, d, dW, db);
     VG_CHECK_LAUNCH("k_conv_bwd_weight");
     return VESPER_OK;
+}
+
+// Shared memory of the 8-channel kernels (two planes of features; the query side of
+// the gradient also keeps its lists), or 0 where it does not fit (sides above 18;
+// those take the general kernels).
+static size_t score8_smem(int d, int lists) {
+    if (d > 31) return 0;   // int16 voxel indices
+    const size_t n = (size_t)d * d * d;
+    const size_t b = 2 * (n + 1) * sizeof(float4) +
+                     lists * (kS8Own * kS8Threads * sizeof(int) + ((n + 7) & ~(size_t)7) * sizeof(int16_t));
+    return b + 4096 <= (size_t)smem_limit() ? b : 0;
+}
+// Rotations per block: whole groups of kS8Rot, about `blocks` blocks in all.
+static int score8_chunk(int nrot, int blocks) {
+    const int per = (nrot + blocks - 1) / blocks;
+    return (per + kS8Rot - 1) / kS8Rot * kS8Rot;
 }
 
 extern "C" int vesper_prop_score(const float *ET, const float *EQ, int K, int d, const float *rotmats, int nrot,
@@ -822,6 +1242,15 @@ extern "C" int vesper_prop_score(const float *ET, const float *EQ, int K, int d,
     if (!ET || !EQ || !rotmats || !scores || K < 1 || d < 1 || nrot < 0)
         return fail(VESPER_ERR_INVALID, "prop_score: bad args");
     if (nrot == 0) return VESPER_OK;
+    const size_t sm8 = score8_smem(d, 0);
+    if (K == 8 && sm8) {
+        const int chunk = score8_chunk(nrot, kPropSMs);
+        allow_smem(k_prop_score8, sm8);
+        k_prop_score8<<<(nrot + chunk - 1) / chunk, kS8Threads, sm8, (cudaStream_t)stream>>>(ET, EQ, d, rotmats, nrot,
+                                                                                            chunk, scores);
+        VG_CHECK_LAUNCH("k_prop_score8");
+        return VESPER_OK;
+    }
     k_prop_score<<<nrot, 256, 0, (cudaStream_t)stream>>>(ET, EQ, K, d, rotmats, nrot, scores);
     VG_CHECK_LAUNCH("k_prop_score");
     return VESPER_OK;
@@ -993,6 +1422,38 @@ extern "C" int vesper_prop_score_bwd(const float *ET, const float *EQ, int K, in
     vesper_prop_score_bwd_workspace(K, d, &need);
     if (!workspace || workspace_bytes < need) return fail(VESPER_ERR_WORKSPACE, "prop_score_bwd: workspace");
     cudaStream_t st = (cudaStream_t)stream;
+    const size_t sm8t = score8_smem(d, 0), sm8q = score8_smem(d, 1);
+    if (K == 8 && sm8t && sm8q) {
+        // slots of the partial gradients (one per chunk of rotations), then the source
+        // table of as many rotations as the workspace holds: groups of equal size
+        const int parts = (n + kS8Own * kS8Threads - 1) / (kS8Own * kS8Threads);
+        const int slots = std::min(nrot, std::max(1, kPropSMs / parts)), ns = (n + 7) & ~7;
+        const size_t used = ((size_t)slots * 16 * n * sizeof(float) + 255) & ~(size_t)255;
+        const int fit = (int)std::min<size_t>((need - used) / (ns * sizeof(int16_t)), (size_t)nrot);
+        const int groups = (nrot + fit - 1) / fit, per_group = (nrot + groups - 1) / groups;
+        int16_t *table = (int16_t *)((char *)workspace + used);
+        allow_smem(k_prop_bwd_t8, sm8t);
+        const size_t sm4 = score8_smem(d, 4), sm2 = score8_smem(d, 2);
+        auto q8 = sm4 ? k_prop_bwd_q8<4> : sm2 ? k_prop_bwd_q8<2> : k_prop_bwd_q8<1>;
+        const size_t smq = sm4 ? sm4 : sm2 ? sm2 : sm8q;
+        allow_smem(q8, smq);
+        for (int r0 = 0; r0 < nrot; r0 += per_group) {
+            const int rn = std::min(per_group, nrot - r0), chunk = (per_group + slots - 1) / slots;
+            k_prop_sources<<<(rn + kS8Rot - 1) / kS8Rot, kSrcThreads, 0, st>>>(d, ns, rotmats + (size_t)r0 * 9, rn, table);
+            VG_CHECK_LAUNCH("k_prop_sources");
+            k_prop_bwd_t8<<<dim3((n + kT8Own * kS8Threads - 1) / (kT8Own * kS8Threads), slots), kS8Threads, sm8t, st>>>(EQ, d, ns, table, rn, gscores + r0, chunk,
+                                                                         r0 > 0, (float *)workspace);
+            VG_CHECK_LAUNCH("k_prop_bwd_t8");
+            q8<<<dim3(parts, slots), kS8Threads, smq, st>>>(ET, d, ns, table, rn, gscores + r0, chunk, r0 > 0,
+                                                            (float *)workspace);
+            VG_CHECK_LAUNCH("k_prop_bwd_q8");
+        }
+        const int nchunk = slots;
+        const int len8 = K * n;
+        k_sum_parts<<<(2 * len8 + 255) / 256, 256, 0, st>>>((const float *)workspace, nchunk, len8, gET, gEQ);
+        VG_CHECK_LAUNCH("k_sum_parts");
+        return VESPER_OK;
+    }
     allow_smem(k_prop_score_bwd, sm);
     for (int k0 = 0; k0 < K; k0 += kc) {
         k_prop_score_bwd<<<nblk, 256, sm, st>>>(ET, EQ, K, k0, kc, d, rotmats, nrot, gscores, chunk,

@@ -133,8 +133,8 @@ class ProposalNet:
 
     def loss_and_grad(self, fT, fQ, mats, q, tau):
         """Accumulate the gradients of one pair; returns the loss tensor."""
-        aT = self.encode(fT)
-        aQ = self.encode(fQ)
+        both = self.encode(torch.stack([fT, fQ]), nmap=2)     # one launch per layer for the two maps
+        aT, aQ = [a[0] for a in both], [a[1] for a in both]
         s = self.score(aT[-1], aQ[-1], mats)
         loss = torch.zeros(1, dtype=torch.float32, device=self.dev.device)
         gs = torch.empty_like(s)
