@@ -12,10 +12,35 @@
 namespace vg {
 
 // ---------------------------------------------------------------------------
-// Pass A for sides up to 32 with whole lines in registers, one x plane per CTA:
+// Pass A for sides up to 32 with whole lines in registers, a few x planes per CTA:
 // the gather, then one packed z line per thread (DFT + unpack in registers),
 // then one y column per thread (DFT in registers, straight to S).
-constexpr int kLineAThreads = 64;   // measured: 64 threads, 1 plane beat 128 and 256 threads, 2 planes
+// Several channels: one plane on 64 threads (measured at side 30, 3 channels: 0.157 us
+// per rotation, 0.182 with 2 planes on 96 threads, although those leave fewer idle;
+// side 32 0.199 and 0.265 with 5 planes).  One channel has 16 lines a plane, so there
+// the fewest idle threads over both phases and the last CTA's planes decide, up to 128
+// threads (side 30: 0.135 -> 0.125 us).
+struct LineShape {
+    int planes, threads;
+};
+template <int SRC, int D>
+__host__ __device__ constexpr LineShape line_a_shape() {
+    constexpr int C = src_nch<SRC>(), NP = (D + 1) / 2, H = D / 2 + 1;
+    LineShape best{1, 64};
+    if (C > 1) return best;
+    long long bn = 0, bd = 1;   // used over held thread slots
+    for (int p = 1; p <= 6; ++p)
+        for (int t = 64; t <= 128; t += 32) {
+            const long long used = (long long)D * C * (NP + H);
+            const long long held = (long long)((D + p - 1) / p) * t * ((p * C * NP + t - 1) / t + (p * C * H + t - 1) / t);
+            if (used * bd > bn * held) {
+                bn = used;
+                bd = held;
+                best = LineShape{p, t};
+            }
+        }
+    return best;
+}
 
 template <int D>
 struct LineGeom {
@@ -25,28 +50,29 @@ struct LineGeom {
 };
 template <int SRC, int D>
 __host__ __device__ constexpr size_t smem_ra_line() {
-    return ((size_t)src_nch<SRC>() * LineGeom<D>::PS + D) * sizeof(float2);
+    return ((size_t)line_a_shape<SRC, D>().planes * src_nch<SRC>() * LineGeom<D>::PS + D) * sizeof(float2);
 }
 
-template <int SRC, int D, bool PFA>
+// T: the block's threads (prob mode's two kinds of channels share a launch).
+template <int SRC, int D, bool PFA, int PL, int T>
 __device__ __forceinline__ void rpass_a_line(const PassA2 &a, int c0) {
     using L = LineGeom<D>;
     constexpr int H = L::H, NP = L::NP, Hp = L::Hp, LS = L::LS, PS = L::PS, NCH = src_nch<SRC>();
     extern __shared__ __align__(16) unsigned char smem[];
-    float2 *buf = (float2 *)smem;   // [NCH][NP][LS]
-    float2 *twn = buf + NCH * PS;
+    float2 *buf = (float2 *)smem;   // [PL][NCH][NP][LS]
+    float2 *twn = buf + PL * NCH * PS;
+    const int x0 = blockIdx.x * PL, b = blockIdx.y, r = a.r0 + b, pn = min(PL, D - x0);
     if constexpr (!PFA) twiddles_n(D, twn);
-    const int x = blockIdx.x, b = blockIdx.y, r = a.r0 + b;
-    if (x == 0 && c0 == 0 && threadIdx.x < a.nscore) a.keys[(size_t)r * a.nscore + threadIdx.x] = 0ull;
+    if (x0 == 0 && c0 == 0 && threadIdx.x < a.nscore) a.keys[(size_t)r * a.nscore + threadIdx.x] = 0ull;
     float F[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) F[i] = __ldg(a.rotmats + (size_t)r * 9 + i);
-    gather_plane<SRC, D, LS, PS, kLineAThreads / 32>(a, F, b, x, buf, [](int z) { return z; });
+    gather_planes<SRC, D, LS, PS, T / 32>(a, F, b, x0, pn, buf, [](int z) { return z; });
     __syncthreads();
     // z: one packed line per thread; DFT and unpack into rows 2p (offset 0)
     // and 2p + 1 (offset Hp) of the line's own storage
-    for (int t = threadIdx.x; t < NCH * NP; t += kLineAThreads) {
-        const int p = t % NP, c = t / NP;
+    for (int t = threadIdx.x; t < pn * NCH * NP; t += T) {
+        const int p = t % NP, c = t / NP;   // c: plane and channel
         float2 *line = buf + c * PS + p * LS;
         float2 v[D];
 #pragma unroll
@@ -62,31 +88,83 @@ __device__ __forceinline__ void rpass_a_line(const PassA2 &a, int c0) {
         }
     }
     __syncthreads();
-    // y: one column (channel, kz) per thread -> S rows ky
-    for (int t = threadIdx.x; t < NCH * H; t += kLineAThreads) {
-        const int kz = t % H, c = t / H;
-        const float2 *pln = buf + c * PS + kz;
+    // y: one column (plane, channel, kz) per thread -> S rows ky
+    for (int t = threadIdx.x; t < pn * NCH * H; t += T) {
+        const int kz = t % H, pc = t / H, pl = pc / NCH, c = pc - pl * NCH;
+        const float2 *pln = buf + pc * PS + kz;
         float2 v[D];
 #pragma unroll
         for (int y = 0; y < D; ++y) v[y] = pln[(y >> 1) * LS + (y & 1) * Hp];
         line_dft<D, D, false, PFA, true>(v, twn);   // largest prime power first (faster here)
-        float2 *dst = a.S + (((size_t)b * a.nch + c0 + c) * D + x) * (size_t)D * H + kz;
+        float2 *dst = a.S + (((size_t)b * a.nch + c0 + c) * D + x0 + pl) * (size_t)D * H + kz;
 #pragma unroll
         for (int ky = 0; ky < D; ++ky) dst[(size_t)ky * H] = v[ky];
     }
 }
 
+// At most 128 registers a thread (8 CTAs of 64 threads per SM).
 template <int SRC, int D, bool PFA>
-__global__ void __launch_bounds__(kLineAThreads, 8) k_rpass_a_line(const PassA2 a) {
-    rpass_a_line<SRC, D, PFA>(a, 0);
+__global__ void __launch_bounds__(line_a_shape<SRC, D>().threads, 512 / line_a_shape<SRC, D>().threads)
+    k_rpass_a_line(const PassA2 a) {
+    constexpr LineShape s = line_a_shape<SRC, D>();
+    rpass_a_line<SRC, D, PFA, s.planes, s.threads>(a, 0);
 }
 // prob mode: the vector channels and the probability channels in CTAs of their own
 template <int D, bool PFA>
-__global__ void __launch_bounds__(kLineAThreads, 8) k_rpass_a_line_prob(const PassA2 a) {
+__global__ void __launch_bounds__(64, 8) k_rpass_a_line_prob(const PassA2 a) {
     if (blockIdx.z == 0)
-        rpass_a_line<kSrcVec, D, PFA>(a, 0);
+        rpass_a_line<kSrcVec, D, PFA, 1, 64>(a, 0);
     else
-        rpass_a_line<kSrcProb, D, PFA>(a, 3);
+        rpass_a_line<kSrcProb, D, PFA, 1, 64>(a, 3);
+}
+
+// A whole line's DFT in registers with the arithmetic of the two register steps
+// (vesper_tilepass.cuh, PFA): N1 points, twiddles, N2 points, or the inverse's
+// opposite order.  For the passes whose sides up to 32 were two-step kernels.
+template <int N1, int N2, bool INV>
+__device__ __forceinline__ void line_dft_two(float2 *v, const float2 *twn) {
+    constexpr int D = N1 * N2;
+    float2 w[D];   // [j2][k1]
+    if constexpr (!INV) {
+#pragma unroll
+        for (int j2 = 0; j2 < N2; ++j2) {
+#pragma unroll
+            for (int j1 = 0; j1 < N1; ++j1) w[N1 * j2 + j1] = v[j2 + N2 * j1];
+            rdft<N1, false>(w + N1 * j2);
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1)
+                if (k1 && j2) w[N1 * j2 + k1] = cmul(w[N1 * j2 + k1], twn[j2 * k1]);
+        }
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) {
+        float2 u[N2];
+#pragma unroll
+        for (int i = 0; i < N2; ++i) u[i] = INV ? v[k1 + N1 * i] : w[N1 * i + k1];
+        rdft<N2, INV>(u);
+#pragma unroll
+        for (int i = 0; i < N2; ++i) {
+            if constexpr (INV)
+                w[N1 * i + k1] = (k1 && i) ? cmulc(u[i], twn[i * k1]) : u[i];
+            else
+                v[k1 + N1 * i] = u[i];
+        }
+    }
+    if constexpr (INV) {
+#pragma unroll
+        for (int j2 = 0; j2 < N2; ++j2) {
+            rdft<N1, true>(w + N1 * j2);
+#pragma unroll
+            for (int j1 = 0; j1 < N1; ++j1) v[j2 + N2 * j1] = w[N1 * j2 + j1];
+        }
+    }
+}
+template <int N1, int N2, bool INV, bool PFA, bool TWO>
+__device__ __forceinline__ void line_dft_as(float2 *v, const float2 *twn) {
+    if constexpr (TWO)
+        line_dft_two<N1, N2, INV>(v, twn);
+    else
+        line_dft<N1 * N2, N1 * N2, INV, PFA>(v, twn);
 }
 
 // ---------------------------------------------------------------------------
@@ -96,11 +174,11 @@ __global__ void __launch_bounds__(kLineAThreads, 8) k_rpass_a_line_prob(const Pa
 // then the inverse x DFT of the sum straight to U.  No shared memory.
 constexpr int kLineBThreads = 64;  // fewer idle threads in the last CTA of each rotation (measured: 64 beat 128, 256)
 
-template <int NCH, int D, bool PFA>
+template <int NCH, int N1, int N2, bool PFA, bool TWO>
 __device__ __forceinline__ void rpass_b_line(const PassB2 &a, int c0, int grp) {
-    constexpr int H = D / 2 + 1, dH = D * H;
-    __shared__ float2 twn[PFA ? 1 : D];
-    if constexpr (!PFA) {
+    constexpr int D = N1 * N2, H = D / 2 + 1, dH = D * H;
+    __shared__ float2 twn[PFA && !TWO ? 1 : D];
+    if constexpr (!PFA || TWO) {
         twiddles_n(D, twn);
         __syncthreads();
     }
@@ -115,27 +193,27 @@ __device__ __forceinline__ void rpass_b_line(const PassB2 &a, int c0, int grp) {
         float2 v[D];
 #pragma unroll
         for (int x = 0; x < D; ++x) v[x] = src[(size_t)(c * D + x) * dH];
-        line_dft<D, D, false, PFA>(v, twn);
+        line_dft_as<N1, N2, false, PFA, TWO>(v, twn);
         const float2 *T = a.T + (size_t)(c0 + c) * D * dH + j;
 #pragma unroll
         for (int k = 0; k < D; ++k) acc[k] = cadd(acc[k], cmul(T[(size_t)k * dH], v[k]));
     }
-    line_dft<D, D, true, PFA>(acc, twn);
+    line_dft_as<N1, N2, true, PFA, TWO>(acc, twn);
     float2 *dst = a.U + ((size_t)b * a.ngrp + grp) * D * dH + j;
 #pragma unroll
     for (int x = 0; x < D; ++x) dst[(size_t)x * dH] = acc[x];
 }
 
-template <int NCH, int D, bool PFA>
+template <int NCH, int N1, int N2, bool PFA>
 __global__ void __launch_bounds__(kLineBThreads) k_rpass_b_line(const PassB2 a) {
-    rpass_b_line<NCH, D, PFA>(a, 0, 0);
+    rpass_b_line<NCH, N1, N2, PFA, false>(a, 0, 0);
 }
-template <int D, bool PFA>
+template <int N1, int N2, bool PFA>
 __global__ void __launch_bounds__(kLineBThreads) k_rpass_b_line_prob(const PassB2 a) {
     if (blockIdx.z == 0)
-        rpass_b_line<3, D, PFA>(a, 0, 0);
+        rpass_b_line<3, N1, N2, PFA, PFA>(a, 0, 0);
     else
-        rpass_b_line<4, D, PFA>(a, 3, 1);
+        rpass_b_line<4, N1, N2, PFA, PFA>(a, 3, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -147,32 +225,41 @@ __global__ void __launch_bounds__(kLineBThreads) k_rpass_b_line_prob(const PassB
 // dropped), inverse DFT (real part row 2p, imaginary part row 2p + 1), the
 // scores' first-index argmax keys; one barrier between the phases.  With
 // several planes per CTA both phases keep most threads busy.
-// Used where 4 planes divide the side (measured: side 28 0.078 -> 0.056 us per
-// rotation, side 32 0.096 -> 0.079 against the two-step pass C; at side 30 it
-// took 0.104-0.111 with 2 to 6 planes per CTA against the two-step's 0.093, so
-// side 30 keeps the two-step kernel).  Threads: the y phase's columns rounded
-// up to whole warps.
-template <int D> __host__ __device__ constexpr int line_c_planes() { return 4; }
-template <int D> __host__ __device__ constexpr bool line_c_used() { return D <= 32 && D % line_c_planes<D>() == 0; }
-template <int D> __host__ __device__ constexpr int line_c_threads() {
-    return (line_c_planes<D>() * (D / 2 + 1) + 31) / 32 * 32 > 128 ? 128
-                                                                   : (line_c_planes<D>() * (D / 2 + 1) + 31) / 32 * 32;
+// Row pairs sit 2 H + 1 elements apart: lanes of the z phase run over row pairs, and
+// with a stride of 2 H, 32 at side 30, all of them fell in one bank.
+// Planes: the divisor of D with the fewest idle threads over both phases (a column
+// per thread, rounded up to whole warps, at most 128).  Microseconds per rotation,
+// mode V: side 30 0.065 (2 planes; 0.092 for the two-step kernel with block
+// barriers between its steps), side 28 0.057 (4), side 32 0.080 (4; 0.104 with 7
+// planes on 128 threads, although those leave fewer idle).
+template <int D> __host__ __device__ constexpr bool line_c_used() { return D <= 32; }
+template <int D> __host__ __device__ constexpr LineShape line_c_shape() {
+    constexpr int NP = (D + 1) / 2, H = D / 2 + 1;
+    LineShape best{1, 32};
+    for (int p = 1; p <= D; ++p) {
+        const int t = (p * H + 31) / 32 * 32;
+        if (D % p == 0 && t <= 128 && p * (NP + H) * best.threads > best.planes * (NP + H) * t) best = LineShape{p, t};
+    }
+    return best;
 }
+template <int D> __host__ __device__ constexpr int line_c_planes() { return line_c_shape<D>().planes; }
+template <int D> __host__ __device__ constexpr int line_c_threads() { return line_c_shape<D>().threads; }
 
 template <int D, int PL>
 __host__ __device__ constexpr size_t smem_rc_line() {
-    return ((size_t)PL * D * (D / 2 + 1) + D) * sizeof(float2) + 2 * sizeof(unsigned long long);
+    return ((size_t)PL * ((D + 1) / 2) * (2 * (D / 2 + 1) + 1) + D + 1) * sizeof(float2) + 2 * sizeof(unsigned long long);
 }
 
-template <int D, bool PFA>
-__global__ void __launch_bounds__(line_c_threads<D>()) k_rpass_c_line(const PassC2 a) {
-    constexpr int H = D / 2 + 1, NP = (D + 1) / 2, PL = line_c_planes<D>();
+template <int N1, int N2, bool PFA>
+__global__ void __launch_bounds__(line_c_threads<N1 * N2>()) k_rpass_c_line(const PassC2 a) {
+    constexpr int D = N1 * N2, H = D / 2 + 1, NP = (D + 1) / 2, PL = line_c_planes<D>(), LS = 2 * H + 1;
+    constexpr bool TWO = PFA && D % 4 != 0;
     extern __shared__ __align__(16) unsigned char smem[];
-    float2 *rows = (float2 *)smem;   // [PL][D][H]
-    unsigned long long *red = (unsigned long long *)(rows + (size_t)PL * D * H);   // [2]
+    float2 *rows = (float2 *)smem;   // [PL][NP][LS]
+    unsigned long long *red = (unsigned long long *)(rows + (size_t)PL * NP * LS);   // [2]
     const int x0 = blockIdx.x * PL, b = blockIdx.y, r = a.r0 + b;
     float2 *twn = (float2 *)(red + 2);
-    if constexpr (!PFA) {
+    if constexpr (!PFA || TWO) {
         twiddles_n(D, twn);
         __syncthreads();
     }
@@ -185,10 +272,10 @@ __global__ void __launch_bounds__(line_c_threads<D>()) k_rpass_c_line(const Pass
         float2 v[D];
 #pragma unroll
         for (int ky = 0; ky < D; ++ky) v[ky] = src[(size_t)ky * H];
-        line_dft<D, D, true, PFA>(v, twn);
-        float2 *dst = rows + (size_t)pl * D * H + kz;
+        line_dft_as<N1, N2, true, PFA, TWO>(v, twn);
+        float2 *dst = rows + (size_t)pl * NP * LS + kz;
 #pragma unroll
-        for (int y = 0; y < D; ++y) dst[(size_t)y * H] = v[y];
+        for (int y = 0; y < D; ++y) dst[(y >> 1) * LS + (y & 1) * H] = v[y];
     }
     __syncthreads();
     // z: row pairs (2p, 2p + 1), inverse complex DFT, scores
@@ -196,7 +283,7 @@ __global__ void __launch_bounds__(line_c_threads<D>()) k_rpass_c_line(const Pass
     for (int t = threadIdx.x; t < PL * NP; t += blockDim.x) {
         const int pl = t / NP, p = t - pl * NP, x = x0 + pl, y = 2 * p;
         if (x >= D) continue;
-        const float2 *r0 = rows + ((size_t)pl * D + y) * H;
+        const float2 *r0 = rows + (pl * NP + p) * LS;
         const bool hb = y + 1 < D;
         const float2 *r1 = r0 + H;
         float2 u[D];
@@ -211,7 +298,7 @@ __global__ void __launch_bounds__(line_c_threads<D>()) k_rpass_c_line(const Pass
                 u[k] = make_float2(A.x + B.y, B.x - A.y);
             }
         }
-        line_dft<D, D, true, PFA>(u, twn);
+        line_dft_as<N1, N2, true, PFA, TWO>(u, twn);
         const uint32_t base = (uint32_t)((x * D + y) * D);
 #pragma unroll
         for (int z = 0; z < D; ++z) {
@@ -261,7 +348,8 @@ struct RegSide {
         if constexpr (kLine) {
             constexpr size_t sm = smem_ra_line<SRC, D>();
             allow_smem(k_rpass_a_line<SRC, D, PFA>, sm);
-            k_rpass_a_line<SRC, D, PFA><<<dim3(D, nb), kLineAThreads, sm, st>>>(p);
+            constexpr LineShape sh = line_a_shape<SRC, D>();
+            k_rpass_a_line<SRC, D, PFA><<<dim3((D + sh.planes - 1) / sh.planes, nb), sh.threads, sm, st>>>(p);
         } else {
             constexpr size_t sm = smem_ta<SRC, N1, N2>();
             allow_smem(k_tpass_a<SRC, N1, N2, PFA>, sm);
@@ -270,9 +358,9 @@ struct RegSide {
     }
     static void a_prob(int nb, cudaStream_t st, const PassA2 &p) {
         if constexpr (kLine) {
-            constexpr size_t sm = smem_ra_line<kSrcProb, D>();
+            constexpr size_t sm = (4 * LineGeom<D>::PS + D) * sizeof(float2);
             allow_smem(k_rpass_a_line_prob<D, PFA>, sm);
-            k_rpass_a_line_prob<D, PFA><<<dim3(D, nb, 2), kLineAThreads, sm, st>>>(p);
+            k_rpass_a_line_prob<D, PFA><<<dim3(D, nb, 2), 64, sm, st>>>(p);
         } else {
             constexpr size_t sm = smem_ta<kSrcProb, N1, N2>();
             allow_smem(k_tpass_a_prob<N1, N2, PFA>, sm);
@@ -282,7 +370,7 @@ struct RegSide {
     template <int NCH>
     static void b(int nb, cudaStream_t st, const PassB2 &p) {
         if constexpr (kLine) {
-            k_rpass_b_line<NCH, D, PFA>
+            k_rpass_b_line<NCH, N1, N2, PFA>
                 <<<dim3((D * H + kLineBThreads - 1) / kLineBThreads, nb), kLineBThreads, 0, st>>>(p);
         } else {
             constexpr int nbx = (D * H + tb_cols<N1>() - 1) / tb_cols<N1>();
@@ -294,7 +382,7 @@ struct RegSide {
     }
     static void b_prob(int nb, cudaStream_t st, const PassB2 &p) {
         if constexpr (kLine) {
-            k_rpass_b_line_prob<D, PFA>
+            k_rpass_b_line_prob<N1, N2, PFA>
                 <<<dim3((D * H + kLineBThreads - 1) / kLineBThreads, nb, 2), kLineBThreads, 0, st>>>(p);
         } else {
             constexpr int nbx = (D * H + tb_cols<N1>() - 1) / tb_cols<N1>();
@@ -315,8 +403,8 @@ struct RegSide {
         if constexpr (line_c_used<D>()) {
             constexpr int PL = line_c_planes<D>();
             constexpr size_t sm = smem_rc_line<D, PL>();
-            allow_smem(k_rpass_c_line<D, PFA>, sm);
-            k_rpass_c_line<D, PFA><<<dim3((D + PL - 1) / PL, nb), line_c_threads<D>(), sm, st>>>(p);
+            allow_smem(k_rpass_c_line<N1, N2, PFA>, sm);
+            k_rpass_c_line<N1, N2, PFA><<<dim3((D + PL - 1) / PL, nb), line_c_threads<D>(), sm, st>>>(p);
         } else {
             tc<1, 1>(nb, st, p);
         }

@@ -105,7 +105,7 @@ __device__ __forceinline__ void store_pair(float2 *at, int p, int z, float v0, f
 // buf[c][line][pos(z)].  Lanes cover 4 lines x 8 z at a time, so a warp's source voxels
 // share cache lines in all three directions.  A voxel with one candidate row per
 // axis is one load (its position's x and y terms are kept per row); the voxels
-// of an odd side's middle index (3 D^2 of D^3) are left to gather_plane.
+// of an odd side's middle index (3 D^2 of D^3) are left to gather_planes.
 template <int SRC, int D, int LS, int CS, class Pos>
 __device__ __forceinline__ void gather_tile(const PassA2 &a, const float (&F)[9], int b, int x, int pt, float2 *buf,
                                             Pos pos) {
@@ -199,13 +199,14 @@ __device__ __forceinline__ void gather_tile(const PassA2 &a, const float (&F)[9]
     }
 }
 
-// Gather of plane x by a CTA of NW warps, each into tiles of its own; on an odd
-// side the voxels of the middle index are shared out over the whole CTA first
-// (2 D - 1 of them, or all of the middle plane and the row that its last line
-// lacks).  Tile pt is ready after a warp
-// barrier on even sides, after a block barrier on odd ones.
+// Gather of pn planes from x0 by a CTA of NW warps, each into tiles of its own (plane
+// stride: the source's channels times CS); on an odd side the voxels of the middle
+// index are shared out over the whole CTA first (2 D - 1 of a plane, or all of the
+// middle plane and the row that its last line lacks).  Ready after a block barrier.
 template <int SRC, int D, int LS, int CS, int NW, class Pos>
-__device__ __forceinline__ void gather_plane(const PassA2 &a, const float (&F)[9], int b, int x, float2 *buf, Pos pos) {
+__device__ __forceinline__ void gather_planes(const PassA2 &a, const float (&F)[9], int b, int x0, int pn, float2 *buf,
+                                              Pos pos) {
+    constexpr int NCH = src_nch<SRC>(), TP = ((D + 1) / 2 + 3) / 4;
     if constexpr (SRC == kSrcVec) {
         // a matrix that is not finite puts no voxel on the grid; its product with the
         // zeros of the missing voxels must not reach the plane
@@ -213,35 +214,37 @@ __device__ __forceinline__ void gather_plane(const PassA2 &a, const float (&F)[9
 #pragma unroll
         for (int i = 0; i < 9; ++i) finite = finite && fabsf(F[i]) <= 3.4028234e38f;
         if (!finite) {
-            for (int e = threadIdx.x; e < 3 * CS; e += NW * 32) buf[e] = make_float2(0.f, 0.f);
+            for (int e = threadIdx.x; e < pn * 3 * CS; e += NW * 32) buf[e] = make_float2(0.f, 0.f);
             return;
         }
     }
     if constexpr ((D & 1) != 0 && SRC != kSrcPlain) {
-        constexpr int M = (D - 1) / 2, NCH = src_nch<SRC>();
-        const bool mid = x == M;
-#pragma unroll 1
-        for (int e = threadIdx.x; e < (mid ? D * (D + 1) : 2 * D - 1); e += NW * 32) {
-            int y = M, z = e;
-            float o[NCH];
-            if (mid) {
-                y = e / D;
-                z = e % D;
-                sample_mid<SRC, D, true>(a.src, F, x, y, z, o);
-            } else {
-                if (e >= D) {
-                    y = e - D + (e - D >= M);
-                    z = M;
-                }
-                sample_mid<SRC, D, false>(a.src, F, x, y, z, o);
-            }
+        constexpr int M = (D - 1) / 2;
+        auto put = [&](int pl, int y, int z, const float *o) {
 #pragma unroll
-            for (int c = 0; c < NCH; ++c) ((float *)(buf + c * CS + (y >> 1) * LS + pos(z)))[y & 1] = o[c];
+            for (int c = 0; c < NCH; ++c) ((float *)(buf + (pl * NCH + c) * CS + (y >> 1) * LS + pos(z)))[y & 1] = o[c];
+        };
+        float o[NCH];
+#pragma unroll 1
+        for (int e = threadIdx.x; e < pn * (2 * D - 1); e += NW * 32) {
+            const int pl = e / (2 * D - 1), f = e - pl * (2 * D - 1);
+            if (x0 + pl == M) continue;
+            const int y = f < D ? M : f - D + (f - D >= M), z = f < D ? f : M;
+            sample_mid<SRC, D, false>(a.src, F, x0 + pl, y, z, o);
+            put(pl, y, z, o);
         }
-        if (mid) return;
+        if (M >= x0 && M < x0 + pn)
+#pragma unroll 1
+            for (int e = threadIdx.x; e < D * (D + 1); e += NW * 32) {
+                sample_mid<SRC, D, true>(a.src, F, M, e / D, e % D, o);
+                put(M - x0, e / D, e % D, o);
+            }
     }
-    for (int pt = threadIdx.x >> 5; pt < ((D + 1) / 2 + 3) / 4; pt += NW)
-        gather_tile<SRC, D, LS, CS>(a, F, b, x, pt, buf, pos);
+    for (int pt = threadIdx.x >> 5; pt < pn * TP; pt += NW) {
+        const int pl = pt / TP, x = x0 + pl;
+        if ((D & 1) != 0 && SRC != kSrcPlain && x == (D - 1) / 2) continue;
+        gather_tile<SRC, D, LS, CS>(a, F, b, x, pt - pl * TP, buf + pl * NCH * CS, pos);
+    }
 }
 
 }  // namespace vg

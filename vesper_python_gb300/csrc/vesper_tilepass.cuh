@@ -87,7 +87,7 @@ __device__ __forceinline__ void tpass_a(const PassA2 &a, int c0) {
     float F[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) F[i] = __ldg(a.rotmats + (size_t)r * 9 + i);
-    gather_plane<SRC, D, LS, CS, NW>(a, F, b, x, buf, [](int z) { return G::pos(z); });
+    gather_planes<SRC, D, LS, CS, NW>(a, F, b, x, 1, buf, [](int z) { return G::pos(z); });
     __syncthreads();
     for (int pt = warp; pt < G::TP; pt += NW) {
         // z step 1, in place: items (c, j2, line), line fastest
