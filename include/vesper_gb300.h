@@ -165,7 +165,9 @@ int vesper_target_spectra(const double *data, const float *vec, const float *pro
  *             translation
  *   nscore = vesper_search_nscore(mode, mix != NULL): 1 for V/O/C/P/L;
  *            prob: {vec, prob} without mix, {vec, prob, mixed} with mix.
- *   batch     rotations resident per pipeline step (0 = library default)
+ *   batch     rotations resident per pipeline step (0 = library default: up to
+ *             256 rotations or 1 GiB of scratch, fewer where the workspace given is
+ *             smaller, down to 64 MB of scratch or one rotation)
  * ------------------------------------------------------------------------- */
 int vesper_search_nscore(int mode, int with_mix);
 int vesper_search_workspace_size(int dim, int mode, int batch, int nrot, size_t *bytes);

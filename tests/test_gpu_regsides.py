@@ -78,3 +78,42 @@ def test_register_passes_equal_radix_stage_passes(dev, mode):
                 assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1]), (mode, d, batch)
             else:
                 assert float((got[0] - ref[0]).abs().max()) <= SCORE_RTOL * float(ref[0].abs().max()), (mode, d)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,d", [("prob", 48), ("VecProduct", 75), ("Laplacian", 50), ("CC", 12)])
+def test_default_batch_fits_the_workspace_given(dev, mode, d):
+    """batch = 0 takes the library's default where the workspace is as large as it asks for, fewer
+    rotations at a time where it is smaller, down to 64 MB of S and U; one smaller still is refused.
+    Every batch gives the same bits."""
+    import ctypes
+
+    from vesper_python_gb300 import _native
+    from vesper_python_gb300 import vesper as vg
+    rng = np.random.default_rng(d)
+    td, tv, tp = (dev.to_dev(a) for a in _fields(rng, d))
+    prob = mode == "prob"
+    spec = vg.target_spectra_device(td, tv, mode, 0.0, probs=tp if prob else None, dev=dev)
+    mats = dev.to_dev(vg.rot_matrices(orc.calc_angle_comb(30.0)[::11]))
+    n, code, ns = int(mats.shape[0]), vg.MODE_CODES[mode], 2 if prob else 1
+    per = ((7 + 2) if prob else 4 if mode == "VecProduct" else 2) * d * d * (d // 2 + 1) * 8
+    base = min(max(1, (64 << 20) // per), 2048)
+    full = _native.size_query("vesper_search_workspace_size", d, code, 0, n)
+    least = _native.size_query("vesper_search_workspace_size", d, code, base, n)
+    assert least <= full
+    ref = vg.search_device(spec, td, tv, mode, 0.0, mats, probs=tp if prob else None, batch=3, dev=dev)
+
+    def call(nbytes):
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev.device)
+        sc = torch.full((n, ns), float("nan"), device=dev.device)
+        ln = torch.full((n, ns), -1, dtype=torch.int32, device=dev.device)
+        p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+        rc = dev.lib.vesper_search(p(spec), p(td), p(tv), p(tp), d, code, 0.0, p(mats), n, None, p(sc), p(ln), 0,
+                                   p(ws), nbytes, dev.stream)
+        torch.cuda.synchronize()
+        return rc, sc, ln
+
+    for nbytes in {full, least, (full + least) // 2}:
+        rc, sc, ln = call(nbytes)
+        assert rc == 0 and torch.equal(sc, ref[0]) and torch.equal(ln, ref[1]), (nbytes, full, least)
+    assert call(least - 4096)[0] == 4

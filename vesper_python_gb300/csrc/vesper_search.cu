@@ -9,8 +9,6 @@
 //   U[b][g][kx][ky][kz] complex64 sum over the group's channels of
 //                       T_c * Q_c after the inverse x pass
 //   keys[r][s]          64-bit (score order bits, ~index) per rotation / score
-// The library's default batch keeps S and U (64 MB) resident in the 129 MB L2
-// across the three passes of a batch.
 #include <algorithm>
 #include <mutex>
 
@@ -48,12 +46,24 @@ static const RegEntry *find_reg(int mode, int d) {
 int vesper_fused_search(int mode, int d, const Src &src, const float *rotmats, const void *spectra, int nrot,
                         int nscore, unsigned long long *keys, cudaStream_t st, int *rc);
 
-static int default_batch(int d, int mode) {
+// Rotations per pipeline step.  base_batch keeps S and U within 64 MB, which small
+// sides need to fill the GPU; default_batch goes on to 256 rotations, or 1 GiB of
+// scratch, since a step of a few rotations leaves most of the SMs' slots idle in
+// its last wave, and that costs more than the trip of S and U through DRAM
+// (microseconds per rotation: prob mode side 64 11.5 with 6 rotations, 8.2 with 128,
+// 8.0 with 256; mode V side 75 9.2 with 9, 5.9 with 128, 5.6 with 256).  No more than
+// there are rotations.
+static size_t batch_bytes(int d, int mode) {
     const size_t H = d / 2 + 1;
-    const size_t per = (size_t)(mode_nch(mode) + mode_ngrp(mode)) * d * d * H * sizeof(float2);
-    const size_t budget = 64ull << 20;
-    int b = (int)std::max<size_t>(1, budget / per);
-    return std::min(b, 2048);
+    return (size_t)(mode_nch(mode) + mode_ngrp(mode)) * d * d * H * sizeof(float2);
+}
+static int base_batch(int d, int mode) {
+    return (int)std::min<size_t>(std::max<size_t>(1, (64ull << 20) / batch_bytes(d, mode)), 2048);
+}
+static int default_batch(int d, int mode, int nrot) {
+    const size_t per = batch_bytes(d, mode) + (mode == VESPER_MODE_LAPLACIAN ? (size_t)d * d * d * sizeof(double) : 0);
+    const int large = (int)std::min<size_t>((1ull << 30) / per, 256), base = base_batch(d, mode);
+    return std::max(base, std::min(large, nrot));
 }
 
 // Shared-memory and thread-count plan of the three passes for side d.
@@ -171,7 +181,7 @@ __global__ void k_laplace(const double *rd, int d, float *out) {
 
 extern "C" int vesper_search_workspace_size(int dim, int mode, int batch, int nrot, size_t *bytes) {
     if (!bytes) return fail(VESPER_ERR_INVALID, "bytes is NULL");
-    if (batch <= 0) batch = default_batch(dim, mode);
+    if (batch <= 0) batch = default_batch(dim, mode, nrot);
     const size_t H = dim / 2 + 1, N = (size_t)dim * dim * dim;
     Carver cv(nullptr, 0);
     cv.take<int>(64);   // status word (tensor-core pass B time-outs)
@@ -199,8 +209,15 @@ static int search_impl(const void *spectra, const double *data, const float *vec
         !scores_out || !lin_out)
         return fail(VESPER_ERR_INVALID, "vesper_search: missing input or output pointer");
     if (mix && mode != VESPER_MODE_PROB) return fail(VESPER_ERR_INVALID, "mix parameters need VESPER_MODE_PROB");
-    if (batch <= 0) batch = default_batch(dim, mode);
     size_t need = 0;
+    if (batch <= 0) {   // a smaller workspace gets a smaller default, down to the base
+        batch = default_batch(dim, mode, nrot);
+        const int base = base_batch(dim, mode);
+        for (; batch > base; batch = std::max(base, batch * 3 / 4)) {
+            vesper_search_workspace_size(dim, mode, batch, nrot, &need);
+            if (workspace_bytes >= need) break;
+        }
+    }
     vesper_search_workspace_size(dim, mode, batch, nrot, &need);
     if (!workspace || workspace_bytes < need)
         return fail(VESPER_ERR_WORKSPACE, "vesper_search: workspace %zu < %zu bytes", workspace_bytes, need);
@@ -430,7 +447,7 @@ extern "C" int vesper_search_profile(const void *spectra, const double *data, co
     for (int p = 0; p < 4; ++p) pass_ms[p] = tm.ms[p];
     int path = 0, launches = 0;
     vesper_search_plan(dim, mode, batch, nrot, opts, &path, &launches);
-    if (batch <= 0) batch = default_batch(dim, mode);
+    if (batch <= 0) batch = default_batch(dim, mode, nrot);
     const int nb = nrot > 0 ? (nrot + batch - 1) / batch : 0;
     pass_launches[0] = path == 2 ? (nrot > 0) : nb;
     pass_launches[1] = pass_launches[2] = path == 2 ? 0 : nb;
@@ -457,7 +474,7 @@ extern "C" int vesper_search_plan(int dim, int mode, int batch, int nrot, const 
             return fail(VESPER_ERR_UNSUPPORTED, "tensor-core pass B: side %d (32 and 64 only)", dim);
         path = 3;
     }
-    if (batch <= 0) batch = default_batch(dim, mode);
+    if (batch <= 0) batch = default_batch(dim, mode, nrot);
     if (path == 3) {   // as the search does: batches of whole waves of tensor-core CTAs
         const int wave = tc_pass_b_wave(dim);
         if (batch > wave) batch = batch / wave * wave;
@@ -533,7 +550,7 @@ extern "C" int vesper_search_static(const void *spectra, const double *data, con
     // the largest pipeline batch (up to the library default) whose scratch fits
     // the array; every batch gives the same results, larger ones fewer launches
     int batch = 1;
-    for (int b = default_batch(dim, mode); b > 1; b = b * 3 / 4) {
+    for (int b = default_batch(dim, mode, nrot); b > 1; b = b * 3 / 4) {
         size_t nb = 0;
         if (vesper_search_workspace_size(dim, mode, b, nrot, &nb) == VESPER_OK && nb <= kStaticScratchBytes) {
             batch = b;
