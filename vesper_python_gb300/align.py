@@ -297,8 +297,22 @@ class Aligner:
             stats, sh = self._global_stage_graph(P, p, mats, nang), None
         else:
             stats, sh = self._global_stage(P, p, mats, nang)
-        device_late = graph and mode not in ("PCC", "CC") and p.A > 5.0 and self.group is None and \
+        # the refinement and rescoring from the device's own results: in the graph form
+        # always, in eager calls where every grid is small.  It searches all N x 27
+        # slots of a pair, about 120 rotations more than the distinct ones, and lets the
+        # pairs' chains of short launches overlap, with no host round trip between the
+        # stages (16 pairs of sides 28 to 32: refinement and rescoring 6.3 -> 2.2 ms,
+        # the whole call 19.9 -> 15.0); at larger sides the 120 rotations cost more than
+        # that gives.
+        late_eager = not graph and max(st.dim for st in P) <= self.LATE_SIDE
+        device_late = (graph or late_eager) and mode not in ("PCC", "CC") and p.A > 5.0 and self.group is None and \
             self._grid_rows(p.A, angle_comb) is not None
+
+        def late_stage():
+            if graph:
+                self._late_stage_graph(P, p, stats, mats)
+            else:
+                self._late_stage(P, p, stats)
 
         def global_results():
             # the global results go to the host while the refinement runs
@@ -316,7 +330,7 @@ class Aligner:
                 # again below
                 zh = self._fetch_start([[zdev]], slot=2)
                 gh = global_results()
-                self._late_stage_graph(P, p, stats, mats)
+                late_stage()
                 zs = self._fetch_finish(zh)[0][0]
             else:
                 zs = zdev.cpu().numpy()
@@ -329,19 +343,19 @@ class Aligner:
                 st.tg.copy_(st.top.to(st.tg.dtype))     # top grid indices, read by the device late stage
             if redo and device_late:
                 gh = global_results()
-                self._late_stage_graph(P, p, stats, mats)
+                late_stage()
             self.proposal_info = {"subset": int(np.ceil(p.proposal_frac * nang)), "z": [float(z) for z in zs],
                                   "fallback": [bool(st.fallback) for st in P]}
         else:
             self.proposal_info = None
         if device_late:
             # refinement and rescoring on the device from the top indices, no
-            # host value in between, replayed as one CUDA graph.  (Eager calls
-            # keep the host-driven refinement below, which searches each
+            # host value in between, replayed as one CUDA graph or launched.  (Other
+            # calls keep the host-driven refinement below, which searches each
             # distinct angle once: fewer rotations, one more host round trip.)
             if gh is None:
                 gh = global_results()
-                self._late_stage_graph(P, p, stats, mats)
+                late_stage()
             return self._finish_device_late(P, p, gh, angle_comb)
         if sh is None:
             sh = stats.cpu().numpy()
@@ -497,6 +511,7 @@ class Aligner:
         return allm, [int(c) for c in counts], dev.to_dev_async(local)
 
     FV_STREAMS = 8
+    LATE_SIDE = 32           # largest grid side whose eager refinement runs from the device's results
     GLOBAL_SIDE = True       # the proposal form's global searches on the side streams too
 
     def _side_streams(self):
