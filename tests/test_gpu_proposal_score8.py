@@ -46,3 +46,24 @@ def test_score8_and_gradients_vs_oracle(dev, d):
     for got, ref, mag, base in ((gT, oT, aT, 0.5), (gQ, oQ, aQ, -0.25)):
         err = np.abs(got.cpu().numpy().reshape(K, n) - (ref + base))
         assert np.all(err <= (mag + abs(base)) * (4 * R + 256) * eps), float((err / (mag + abs(base))).max())
+
+
+@pytest.mark.parametrize("d,nrot", [(1, 3), (2, 5), (7, 16), (10, 33), (15, 700), (18, 700)])
+def test_score8_sums_are_the_general_kernels(dev, d, nrot):
+    """A ninth channel of zeros takes the general kernel and adds nothing: the same bits, infinities in features
+    that no rotation reaches included."""
+    from vesper_python_gb300 import proposal as P
+    from vesper_python_gb300 import vesper as vg
+    net = P.ProposalNet(dev, seed=1)
+    g = torch.Generator().manual_seed(d)
+    t, q = (torch.randn((8, d, d, d), generator=g).to(dev.device) for _ in range(2))
+    angles = orc.calc_angle_comb(10.0)
+    mats = dev.to_dev(vg.rot_matrices(angles[::max(1, len(angles) // nrot)][:nrot]))
+    for bad in (False, True):
+        if bad:
+            t[3, 0, 0, 0] = float("inf")
+            q[3, -1, -1, -1] = float("inf")
+        ninth = [torch.cat([a, torch.zeros_like(a[:1])]).contiguous() for a in (t, q)]
+        a, b = net.score(t, q, mats), net.score(*ninth, mats)
+        assert torch.equal(a.view(torch.int32)[~a.isnan()], b.view(torch.int32)[~b.isnan()])
+        assert torch.equal(a.isnan(), b.isnan())
