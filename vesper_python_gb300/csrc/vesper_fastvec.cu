@@ -51,9 +51,13 @@ struct AxisTables {
     double *wp;      // [3][WB][d]  weight * (stp + k)
     float2 *wf;      // [3][WB][d]  w as a float-float pair (hi, lo)
     float2 *wpf;     // [3][WB][d]  wp as a pair
-    int *plane;      // [S0] source plane xp holds a non-zero value (written by the z stage)
-    int *list;       // [S0 S1] source rows holding a non-zero value (float-float z stage)
-    int *nlist;      // [1] their count
+    // float-float stages, written by k_fvf_scan
+    int *rlo, *rhi;          // [S0] first and last row of plane xp that holds a non-zero value (rhi -1: none)
+    int *list;               // [S0 S1] the rows that do, any order
+    unsigned char *rowf;     // [S0 S1] 1 where a row does
+    unsigned char *need;     // [d d] 1 where column (y, z) has a voxel that passes the skip tests
+    int *voxels;             // [d^3] those voxels, any order
+    int *count;              // [4] rows listed, voxels listed, first and last plane with a row
 };
 
 struct FvGeom {
@@ -69,9 +73,14 @@ __global__ void k_fv_tables(const FvGeom g, AxisTables t) {
     const int i = blockIdx.x;
     const int a = blockIdx.y;
     if (i >= g.d) return;
-    if (a == 0)   // clear the plane flags: block i takes planes i*128 + tid + m*128*d
-        for (int xp = i * blockDim.x + threadIdx.x; xp < g.S[0]; xp += g.d * blockDim.x) t.plane[xp] = 0;
-    if (a == 0 && i == 0 && threadIdx.x == 0) *t.nlist = 0;
+    if (a == 0)   // clear the lists: block i takes planes i*128 + tid + m*128*d
+        for (int xp = i * blockDim.x + threadIdx.x; xp < g.S[0]; xp += g.d * blockDim.x) {
+            t.rlo[xp] = g.S[1];
+            t.rhi[xp] = -1;
+        }
+    if (a == 1)
+        for (int z = threadIdx.x; z < g.d; z += blockDim.x) t.need[i * g.d + z] = 0;
+    if (a == 2 && i == 0 && threadIdx.x < 4) t.count[threadIdx.x] = threadIdx.x == 2 ? g.S[0] : threadIdx.x == 3 ? -1 : 0;
     // (xyz_arr * dest_xwidth + dest_orig - src_orig) / src_xwidth
     double p = __dmul_rn((double)i, g.dw);
     p = __dadd_rn(p, g.dorig[a]);
@@ -299,329 +308,334 @@ __global__ void __launch_bounds__(256) k_fv_x(const float *src, const FvGeom g, 
 
 // ---- float-float stages ---------------------------------------------------------
 
-// stage 1a: list the source rows (xp, yp) that hold a non-zero value (one warp
-// per row, any order: each row's sums are independent of the others) and mark
-// their planes; an all-zero row's sums are +0.0, as the reference's loop gives,
-// and are written here.
-__global__ void __launch_bounds__(256) k_fvf_rows(const float *src, const FvGeom g, const AxisTables t,
-                                                  float2 *A0, float2 *A1) {
-    const int S1 = g.S[1], S2 = g.S[2], d = g.d;
-    const size_t nrows = (size_t)g.S[0] * S1;
-    const int lane = threadIdx.x & 31;
-    for (size_t row = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < nrows; row += (size_t)gridDim.x * 8) {
-        const float *rp = src + row * S2;
-        bool nz = false;
-        for (int e = lane; e < S2; e += 32) nz |= __ldg(rp + e) != 0.f;
-        if (__any_sync(0xffffffffu, nz)) {
-            if (lane == 0) {
-                t.list[atomicAdd(t.nlist, 1)] = (int)row;
-                t.plane[row / S1] = 1;
-            }
-        } else {
-            for (int z = lane; z < d; z += 32) {
-                A0[row * d + z] = make_float2(0.f, 0.f);
-                A1[row * d + z] = make_float2(0.f, 0.f);
-            }
-        }
-    }
-}
-
-// stage 1b (z).  Block b takes listed rows [b kZRows, (b + 1) kZRows), staged in
-// shared memory with one extra all-zero row, together with the z axis's weight
-// pairs when they fit (SW); each thread sums kFfRows of the rows for one output
-// z, so every weight pair it loads serves kFfRows rows.  Blocks past the list's
-// end return at once.
-constexpr int kZRows = 16;
-constexpr int kFfRows = 2;
-constexpr int kFfBatch = 8;   // band entries loaded per round by the global-load forms
-template <bool SW>
-__global__ void __launch_bounds__(256) k_fvf_z(const float *src, const FvGeom g, const AxisTables t, float2 *A0,
-                                               float2 *A1) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int S2 = g.S[2], d = g.d, WB = g.WB;
-    const int first = blockIdx.x * kZRows;
-    const int nr = min(kZRows, *t.nlist - first);
-    if (nr <= 0) return;   // block-uniform
-    float2 *sw = (float2 *)smem;                          // [WB][d] when SW
-    float2 *swp = sw + (SW ? (size_t)WB * d : 0);         // [WB][d] when SW
-    float *rows = (float *)(swp + (SW ? (size_t)WB * d : 0));   // [kZRows + 1][S2]
-    const float2 *gw = t.wf + (size_t)2 * WB * d, *gwp = t.wpf + (size_t)2 * WB * d;
-    if (SW)
-        for (int e = threadIdx.x; e < WB * d; e += blockDim.x) {
-            sw[e] = __ldg(gw + e);
-            swp[e] = __ldg(gwp + e);
-        }
-#pragma unroll 4
-    for (int e = threadIdx.x; e < (kZRows + 1) * S2; e += blockDim.x) {
-        const int r = e / S2;
-        rows[e] = r < nr ? __ldg(src + (size_t)t.list[first + r] * S2 + (e - r * S2)) : 0.f;
-    }
-    __syncthreads();
-    const int ng = (nr + kFfRows - 1) / kFfRows;
-    const int *stp = t.stp + 2 * d, *len = t.len + 2 * d;
-    const float2 *w = SW ? sw : gw, *wp = SW ? swp : gwp;
-    for (int it = threadIdx.x; it < ng * d; it += blockDim.x) {
-        const int gi = it / d, z = it - gi * d;
-        int off[kFfRows];
-#pragma unroll
-        for (int r = 0; r < kFfRows; ++r) {
-            const int li = gi * kFfRows + r;
-            off[r] = (li < nr ? li : kZRows) * S2 + stp[z];   // row kZRows is all zero
-        }
-        float s0h[kFfRows], s0l[kFfRows], s1h[kFfRows], s1l[kFfRows];
-#pragma unroll
-        for (int r = 0; r < kFfRows; ++r) s0h[r] = s0l[r] = s1h[r] = s1l[r] = 0.f;
-        const int n = len[z];
+// stage 1a.  Blocks below row_blocks list the source rows (xp, yp) that hold a
+// non-zero value (a warp per row; 16-byte loads where VEC) and bound each plane's;
+// the others list the destination voxels that pass the skip tests
+// (VESPER_1_prob_new.py:200-211), mark their columns and zero the rest of the output.
+// Lists in any order: every row's and voxel's sums are independent of the others.
+// Bound by the read of the source (256^3: 67 MB).
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_fvf_scan(const float *src, const FvGeom g, const AxisTables t, int row_blocks,
+                                                  double *data_out, float *data_f32, float *vec_out) {
+    const int S1 = g.S[1], S2 = g.S[2], d = g.d, lane = threadIdx.x & 31;
+    if ((int)blockIdx.x < row_blocks) {
+        // rounds of 64 rows, 8 per warp, so that a block's rows cost a few atomics
+        __shared__ unsigned char flag[64];
+        const size_t nrows = (size_t)g.S[0] * S1;
+        for (size_t row0 = (size_t)blockIdx.x * 64; row0 < nrows; row0 += (size_t)row_blocks * 64) {
 #pragma unroll 2
-        for (int k = 0; k < n; ++k) {
-            const float2 a = w[(size_t)k * d + z], b = wp[(size_t)k * d + z];
-#pragma unroll
-            for (int r = 0; r < kFfRows; ++r) {
-                const float v = rows[off[r] + k];
-                float ph, pl;
-                ff_mul_f(a.x, a.y, v, ph, pl);
-                ff_add(s0h[r], s0l[r], ph, pl);
-                ff_mul_f(b.x, b.y, v, ph, pl);
-                ff_add(s1h[r], s1l[r], ph, pl);
+            for (int q = 0; q < 8; ++q) {
+                const size_t row = row0 + (threadIdx.x >> 5) * 8 + q;
+                const float *rp = src + row * S2;
+                bool nz = false;
+                if (row < nrows) {
+                    if (VEC) {
+#pragma unroll 2
+                        for (int e = lane; e < S2 / 4; e += 32) {
+                            const float4 v = __ldg((const float4 *)rp + e);
+                            nz |= v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f;
+                        }
+                    } else {
+#pragma unroll 4
+                        for (int e = lane; e < S2; e += 32) nz |= __ldg(rp + e) != 0.f;
+                    }
+                }
+                nz = __any_sync(0xffffffffu, nz);
+                if (lane == 0) flag[(threadIdx.x >> 5) * 8 + q] = nz;
             }
-        }
-#pragma unroll
-        for (int r = 0; r < kFfRows; ++r) {
-            const int li = gi * kFfRows + r;
-            if (li < nr) {
-                const size_t o = (size_t)t.list[first + li] * d + z;
-                A0[o] = make_float2(s0h[r], s0l[r]);
-                A1[o] = make_float2(s1h[r], s1l[r]);
+            __syncthreads();
+            if (threadIdx.x < 64) {   // two whole warps
+                const size_t row = row0 + threadIdx.x;
+                const bool nz = flag[threadIdx.x];
+                if (row < nrows) t.rowf[row] = nz;
+                const unsigned m = __ballot_sync(0xffffffffu, nz);
+                int base = 0;
+                if (lane == 0 && m) base = atomicAdd(t.count, __popc(m));
+                base = __shfl_sync(0xffffffffu, base, 0);
+                if (nz) {
+                    t.list[base + __popc(m & ((1u << lane) - 1u))] = (int)row;
+                    const int xp = (int)(row / S1), yp = (int)(row - (size_t)xp * S1);
+                    // the bounds only move outwards: most rows see theirs already there
+                    if (yp < *(volatile int *)(t.rlo + xp)) atomicMin(t.rlo + xp, yp);
+                    if (yp > *(volatile int *)(t.rhi + xp)) atomicMax(t.rhi + xp, yp);
+                    if (xp < *(volatile int *)(t.count + 2)) atomicMin(t.count + 2, xp);
+                    if (xp > *(volatile int *)(t.count + 3)) atomicMax(t.count + 3, xp);
+                }
             }
-        }
-    }
-}
-
-// stage 2 (y).  Block = (z tile of 32, source plane xp, chunk of yc consecutive
-// outputs y); lanes over z, warp w sums outputs y0 + w, y0 + w + 8, ...  The
-// rows of A0 and A1 that the chunk's bands cover (at most rmax, a bound the
-// host derives from the geometry) and the chunk's weight pairs are first copied
-// to shared memory with coalesced loads that are all in flight together; a
-// block whose rows exceed rmax (rmax = 0: the slab does not fit) reads global
-// memory instead, kFfBatch band entries per round.  A plane without a non-zero
-// value gives +0.0.
-__global__ void __launch_bounds__(256) k_fvf_y(const FvGeom g, const AxisTables t, int yc, int rmax,
-                                               const float2 *A0, const float2 *A1, float2 *B0, float2 *B1,
-                                               float2 *B2) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int S1 = g.S[1], d = g.d, WB = g.WB;
-    const int z0 = blockIdx.x * 32, xp = blockIdx.y, y0 = blockIdx.z * yc;
-    const int yn = min(yc, d - y0);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int z = z0 + lane;
-    const int *stp = t.stp + d, *len = t.len + d;
-    const float2 *wf = t.wf + (size_t)WB * d, *wpf = t.wpf + (size_t)WB * d;
-    if (!t.plane[xp]) {
-        for (int e = threadIdx.x; e < yn * 32; e += blockDim.x) {
-            const int zz = z0 + (e & 31), y = y0 + (e >> 5);
-            if (zz < d) {
-                const size_t go = ((size_t)xp * d + y) * d + zz;
-                B0[go] = B1[go] = B2[go] = make_float2(0.f, 0.f);
-            }
+            __syncthreads();
         }
         return;
     }
-    const int r0 = stp[y0];
-    int r1 = r0;
-    for (int y = y0; y < y0 + yn; ++y) r1 = max(r1, stp[y] + len[y]);
-    const bool slab = r1 - r0 <= rmax;   // block-uniform
-    float2 *s0 = (float2 *)smem;            // [rmax][32]
-    float2 *s1 = s0 + (size_t)rmax * 32;    // [rmax][32]
-    float2 *sw = s1 + (size_t)rmax * 32;    // [yc][WB]
-    float2 *swp = sw + (size_t)yc * WB;     // [yc][WB]
-    if (slab) {
-#pragma unroll 4
-        for (int e = threadIdx.x; e < (r1 - r0) * 32; e += blockDim.x) {
-            const int r = e >> 5, zz = z0 + (e & 31);
-            float2 v0 = make_float2(0.f, 0.f), v1 = v0;
-            if (zz < d) {
-                const size_t gi = ((size_t)xp * S1 + r0 + r) * d + zz;
-                v0 = __ldg(A0 + gi);
-                v1 = __ldg(A1 + gi);
-            }
-            s0[e] = v0;
-            s1[e] = v1;
+    const int v = ((int)blockIdx.x - row_blocks) * 256 + threadIdx.x, dd = d * d;
+    bool valid = false;
+    if (v < dd * d) {
+        const int x = v / dd, yz = v - x * dd, y = yz / d, z = yz - y * d;
+        const int ix = t.idx[x], iy = t.idx[d + y], iz = t.idx[2 * d + z];
+        valid = ix >= 0 && iy >= 0 && iz >= 0;
+        if (valid) valid = src[((size_t)ix * S1 + iy) * S2 + iz] != 0.f;
+        if (valid) {
+            t.need[yz] = 1;
+        } else {
+            data_out[v] = 0.0;
+            if (data_f32) data_f32[v] = 0.f;
+            vec_out[3 * (size_t)v] = vec_out[3 * (size_t)v + 1] = vec_out[3 * (size_t)v + 2] = 0.f;
         }
-        for (int e = threadIdx.x; e < yn * WB; e += blockDim.x) {
-            const int yy = e / WB, k = e - yy * WB;
-            sw[e] = __ldg(wf + (size_t)k * d + y0 + yy);
-            swp[e] = __ldg(wpf + (size_t)k * d + y0 + yy);
-        }
-        __syncthreads();
     }
-    for (int yy = wid; yy < yn; yy += 8) {
-        const int y = y0 + yy;
-        const int n = len[y], s = stp[y];
-        float b0h = 0.f, b0l = 0.f, b1h = 0.f, b1l = 0.f, b2h = 0.f, b2l = 0.f;
-        auto term = [&](float2 wy, float2 wyp, float2 v0, float2 v1) {
-            float ph, pl;
-            ff_mul(v0, wy, ph, pl);
-            ff_add(b0h, b0l, ph, pl);
-            ff_mul(v0, wyp, ph, pl);
-            ff_add(b1h, b1l, ph, pl);
-            ff_mul(v1, wy, ph, pl);
-            ff_add(b2h, b2l, ph, pl);
-        };
-        if (slab) {
-            const float2 *a0 = s0 + (size_t)(s - r0) * 32 + lane, *a1 = s1 + (size_t)(s - r0) * 32 + lane;
-            const float2 *w = sw + (size_t)yy * WB, *wp = swp + (size_t)yy * WB;
+    const unsigned m = __ballot_sync(0xffffffffu, valid);
+    int base = 0;
+    if (lane == 0 && m) base = atomicAdd(t.count + 1, __popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (valid) t.voxels[base + __popc(m & ((1u << lane) - 1u))] = v;
+}
+
+// stage 1b (z).  Block b takes listed rows [b kZRows, (b + 1) kZRows): each row's
+// non-zero entries are packed in order into shared memory with the count before
+// every entry, so that a thread, one output z of one row, sums just the non-zero
+// entries of its band (most of a thresholded row is zero, and a zero adds nothing
+// to a pair sum).  The z axis's weight pairs are staged too when they fit (SW).
+// Every entry of the band for two rows per thread took 101 us (256^3 -> 42^3) and 30
+// (128^3 -> 28^3); now 41 and 9.5.
+constexpr int kZRows = 16;
+constexpr int kZThreads = 512;
+constexpr int kFfBatch = 8;    // band entries loaded per round by the y stage from global memory
+constexpr int kXBatch = 16;    // and by the x stage
+struct ZEntry {
+    float v;
+    int e;
+};
+// rows: kZRows, fewer where long source rows would not fit
+__host__ __device__ inline size_t fvf_z_rows_smem(int S2, int rows) {
+    return (size_t)rows * (S2 * sizeof(ZEntry) + (S2 + 1 + 3) / 4 * 4 * sizeof(short));
+}
+template <bool SW>
+__global__ void __launch_bounds__(kZThreads) k_fvf_z(const float *src, const FvGeom g, const AxisTables t, int rows,
+                                                     float2 *A0, float2 *A1) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int S2 = g.S[2], d = g.d, WB = g.WB, CN = (S2 + 1 + 3) / 4 * 4;
+    const int first = blockIdx.x * rows;
+    const int nr = min(rows, t.count[0] - first);
+    if (nr <= 0) return;   // block-uniform
+    ZEntry *ent = (ZEntry *)smem;                                      // [rows][S2]
+    unsigned short *cnt = (unsigned short *)(ent + rows * S2);         // [rows][CN]
+    float2 *sw = (float2 *)(smem + fvf_z_rows_smem(S2, rows));         // [WB][d] when SW
+    float2 *swp = sw + (SW ? (size_t)WB * d : 0);                      // [WB][d] when SW
+    const float2 *gw = t.wf + (size_t)2 * WB * d, *gwp = t.wpf + (size_t)2 * WB * d;
+    if (SW)
+#pragma unroll 4
+        for (int e = threadIdx.x; e < WB * d; e += kZThreads) {
+            sw[e] = __ldg(gw + e);
+            swp[e] = __ldg(gwp + e);
+        }
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < nr; r += kZThreads / 32) {
+        const float *rp = src + (size_t)t.list[first + r] * S2;
+        int n = 0;
+        for (int e0 = 0; e0 < S2; e0 += 32) {
+            const int e = e0 + lane;
+            const float v = e < S2 ? __ldg(rp + e) : 0.f;
+            const unsigned m = __ballot_sync(0xffffffffu, v != 0.f);
+            const int at = n + __popc(m & ((1u << lane) - 1u));
+            if (e < S2) cnt[r * CN + e] = (unsigned short)at;
+            if (v != 0.f) ent[r * S2 + at] = ZEntry{v, e};
+            n += __popc(m);
+        }
+        if (lane == 0) cnt[r * CN + S2] = (unsigned short)n;
+    }
+    __syncthreads();
+    const int *stp = t.stp + 2 * d, *len = t.len + 2 * d;
+    const float2 *w = SW ? sw : gw, *wp = SW ? swp : gwp;
+    for (int it = threadIdx.x; it < nr * d; it += kZThreads) {
+        const int r = it / d, z = it - r * d, s = min(stp[z], S2), n = len[z];
+        const int lo = cnt[r * CN + s], hi = n > 0 ? cnt[r * CN + s + n] : lo;
+        const ZEntry *ep = ent + r * S2;
+        const float2 *wz = w + z - (size_t)s * d, *wpz = wp + z - (size_t)s * d;
+        float s0h = 0.f, s0l = 0.f, s1h = 0.f, s1l = 0.f;
 #pragma unroll 2
-            for (int k = 0; k < n; ++k) term(w[k], wp[k], a0[k * 32], a1[k * 32]);
-        } else if (z < d) {
-            const float2 *w = wf + y, *wp = wpf + y;
-            const float2 *a0 = A0 + ((size_t)xp * S1 + s) * d + z, *a1 = A1 + ((size_t)xp * S1 + s) * d + z;
-            int k = 0;
-            for (; k + kFfBatch <= n; k += kFfBatch) {
-                float2 wy[kFfBatch], wyp[kFfBatch], v0[kFfBatch], v1[kFfBatch];
-#pragma unroll
-                for (int u = 0; u < kFfBatch; ++u) {
-                    const size_t o = (size_t)(k + u) * d;
-                    wy[u] = __ldg(w + o);
-                    wyp[u] = __ldg(wp + o);
-                    v0[u] = __ldg(a0 + o);
-                    v1[u] = __ldg(a1 + o);
-                }
-#pragma unroll
-                for (int u = 0; u < kFfBatch; ++u) term(wy[u], wyp[u], v0[u], v1[u]);
-            }
-            for (; k < n; ++k) {
-                const size_t o = (size_t)k * d;
-                term(__ldg(w + o), __ldg(wp + o), __ldg(a0 + o), __ldg(a1 + o));
-            }
+        for (int i = lo; i < hi; ++i) {
+            const ZEntry q = ep[i];
+            const float2 a = wz[(size_t)q.e * d], b = wpz[(size_t)q.e * d];
+            float ph, pl;
+            ff_mul_f(a.x, a.y, q.v, ph, pl);
+            ff_add(s0h, s0l, ph, pl);
+            ff_mul_f(b.x, b.y, q.v, ph, pl);
+            ff_add(s1h, s1l, ph, pl);
         }
-        if (z < d) {
-            const size_t go = ((size_t)xp * d + y) * d + z;
-            B0[go] = make_float2(b0h, b0l);
-            B1[go] = make_float2(b1h, b1l);
-            B2[go] = make_float2(b2h, b2l);
-        }
+        const size_t o = (size_t)t.list[first + r] * d + z;
+        A0[o] = make_float2(s0h, s0l);
+        A1[o] = make_float2(s1h, s1l);
     }
 }
 
-// stage 3 (x) and each voxel's finish.  Block = (z tile of 32, output y, chunk
-// of xc consecutive outputs x); lanes over z, warp w sums outputs x0 + w, ...,
-// from a shared-memory slab of B0, B1, B2 as in stage 2.
-__global__ void __launch_bounds__(256) k_fvf_x(const float *src, const FvGeom g, const AxisTables t, int xc,
-                                               int rmax, const float2 *B0, const float2 *B1, const float2 *B2,
-                                               double *data_out, float *data_f32, float *vec_out) {
+// stage 2 (y).  Block = (z tile of zw, source plane xp, chunk of yc consecutive
+// outputs y).  The rows of A0 and A1 that the chunk's bands cover, between the
+// plane's first and last row with a non-zero value (at most rmax, a bound the host
+// derives from the geometry), and the chunk's weight pairs are first copied to shared
+// memory with coalesced loads that are all in flight together; a block whose rows
+// exceed rmax (rmax = 0: the slab does not fit) reads global memory instead, kFfBatch
+// band entries per round.  Only the columns that stage 3 will read are computed: the
+// block packs them into a list, and each of a column's three sums has a thread (the
+// sums are long dependent chains: with three a thread the SMs idled).  A plane without a non-zero value
+// gives +0.0, and none before the first such plane or after the last is read.
+// All columns, lanes over tiles of 32 z: 79 us (256^3 -> 42^3) and 22 (128^3 -> 28^3);
+// now 43 and 18.5.
+constexpr int kYThreads = 256;
+__global__ void __launch_bounds__(kYThreads) k_fvf_y(const FvGeom g, const AxisTables t, int zw, int yc, int rmax,
+                                                     const float2 *A0, const float2 *A1, float2 *B0, float2 *B1,
+                                                     float2 *B2) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int d = g.d, WB = g.WB;
-    const int z0 = blockIdx.x * 32, y = blockIdx.y, x0 = blockIdx.z * xc;
-    const int xn = min(xc, d - x0);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int z = z0 + lane;
-    const int *stp = t.stp, *len = t.len;
-    const size_t plane = (size_t)d * d;
-    const int r0 = stp[x0];
-    int r1 = r0;
-    for (int x = x0; x < x0 + xn; ++x) r1 = max(r1, stp[x] + len[x]);
+    __shared__ int ncol;
+    const int S1 = g.S[1], d = g.d, WB = g.WB;
+    const int z0 = blockIdx.x * zw, xp = blockIdx.y, y0 = blockIdx.z * yc;
+    const int yn = min(yc, d - y0), zn = min(zw, d - z0);
+    if (xp < t.count[2] || xp > t.count[3] || zn <= 0) return;   // block-uniform, as below
+    const int *stp = t.stp + d, *len = t.len + d;
+    const float2 *wf = t.wf + (size_t)WB * d, *wpf = t.wpf + (size_t)WB * d;
+    const int plo = t.rlo[xp], phi = t.rhi[xp] + 1;
+    int r0 = S1, r1 = 0;
+    for (int y = y0; y < y0 + yn; ++y) {
+        r0 = min(r0, stp[y]);
+        r1 = max(r1, stp[y] + len[y]);
+    }
+    r0 = max(r0, plo);
+    r1 = max(min(r1, phi), r0);
     const bool slab = r1 - r0 <= rmax;   // block-uniform
-    float2 *s0 = (float2 *)smem;            // [rmax][32] each
-    float2 *s1 = s0 + (size_t)rmax * 32;
-    float2 *s2 = s1 + (size_t)rmax * 32;
-    float2 *sw = s2 + (size_t)rmax * 32;    // [xc][WB]
-    float2 *swp = sw + (size_t)xc * WB;     // [xc][WB]
+    float2 *s0 = (float2 *)smem;            // [rmax][zw]
+    float2 *s1 = s0 + (size_t)rmax * zw;    // [rmax][zw]
+    float2 *sw = s1 + (size_t)rmax * zw;    // [yc][WB]
+    float2 *swp = sw + (size_t)yc * WB;     // [yc][WB]
+    unsigned short *cols = (unsigned short *)(swp + (size_t)yc * WB);   // [yc zw]
+    if (threadIdx.x == 0) ncol = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int c0 = 0; c0 < yn * zw; c0 += kYThreads) {
+        const int c = c0 + threadIdx.x, yy = c / zw, zz = c - yy * zw;
+        const bool on = c < yn * zw && zz < zn && t.need[(y0 + yy) * d + z0 + zz];
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        int base = 0;
+        if (lane == 0 && m) base = atomicAdd(&ncol, __popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (on) cols[base + __popc(m & ((1u << lane) - 1u))] = (unsigned short)c;
+    }
+    __syncthreads();
+    const int nc = ncol;
+    if (nc == 0) return;
     if (slab) {
 #pragma unroll 4
-        for (int e = threadIdx.x; e < (r1 - r0) * 32; e += blockDim.x) {
-            const int r = e >> 5, zz = z0 + (e & 31);
-            float2 v0 = make_float2(0.f, 0.f), v1 = v0, v2 = v0;
-            if (zz < d) {
-                const size_t gi = (size_t)(r0 + r) * plane + (size_t)y * d + zz;
-                v0 = __ldg(B0 + gi);
-                v1 = __ldg(B1 + gi);
-                v2 = __ldg(B2 + gi);
+        for (int e = threadIdx.x; e < (r1 - r0) * zw; e += kYThreads) {
+            const int r = e / zw, zz = e - r * zw;
+            float2 v0 = make_float2(0.f, 0.f), v1 = v0;
+            const size_t row = (size_t)xp * S1 + r0 + r;
+            if (zz < zn && t.rowf[row]) {
+                v0 = __ldg(A0 + row * d + z0 + zz);
+                v1 = __ldg(A1 + row * d + z0 + zz);
             }
             s0[e] = v0;
             s1[e] = v1;
-            s2[e] = v2;
         }
-        for (int e = threadIdx.x; e < xn * WB; e += blockDim.x) {
-            const int xx = e / WB, k = e - xx * WB;
-            sw[e] = __ldg(t.wf + (size_t)k * d + x0 + xx);
-            swp[e] = __ldg(t.wpf + (size_t)k * d + x0 + xx);
+        for (int e = threadIdx.x; e < yn * WB; e += kYThreads) {
+            const int k = e / yn, yy = e - k * yn;
+            sw[yy * WB + k] = __ldg(wf + (size_t)k * d + y0 + yy);
+            swp[yy * WB + k] = __ldg(wpf + (size_t)k * d + y0 + yy);
         }
         __syncthreads();
     }
-    if (z >= d) return;   // no barrier below
-    for (int xx = wid; xx < xn; xx += 8) {
-        const int x = x0 + xx;
-        // skip tests (VESPER_1_prob_new.py:200-211)
-        const int ix = t.idx[x], iy = t.idx[d + y], iz = t.idx[2 * d + z];
-        bool valid = ix >= 0 && iy >= 0 && iz >= 0;
-        if (valid) valid = src[((size_t)ix * g.S[1] + iy) * g.S[2] + iz] != 0.f;
-        float dh = 0.f, dl = 0.f, xh = 0.f, xl = 0.f, yh = 0.f, yl = 0.f, zh = 0.f, zl = 0.f;
-        auto term = [&](float2 wx, float2 wxp, float2 v0, float2 v1, float2 v2) {
+    // item (sum, column), columns fastest: B0 = sum w A0, B1 = sum wp A0, B2 = sum w A1
+    for (int it = threadIdx.x; it < 3 * nc; it += kYThreads) {
+        const int q = it >= 2 * nc ? 2 : it >= nc, col = cols[it - q * nc];
+        const int yy = col / zw, zz = col - yy * zw, y = y0 + yy, z = z0 + zz;
+        const int s = stp[y], k0 = max(0, plo - s), n = min(len[y], phi - s);
+        float bh = 0.f, bl = 0.f;
+        auto term = [&](float2 w, float2 v) {
             float ph, pl;
-            ff_mul(v0, wx, ph, pl);
-            ff_add(dh, dl, ph, pl);
-            ff_mul(v0, wxp, ph, pl);
-            ff_add(xh, xl, ph, pl);
-            ff_mul(v1, wx, ph, pl);
-            ff_add(yh, yl, ph, pl);
-            ff_mul(v2, wx, ph, pl);
-            ff_add(zh, zl, ph, pl);
+            ff_mul(v, w, ph, pl);
+            ff_add(bh, bl, ph, pl);
         };
-        const int n = len[x], s = stp[x];
-        if (valid && slab) {
-            const size_t o = (size_t)(s - r0) * 32 + lane;
-            const float2 *v0 = s0 + o, *v1 = s1 + o, *v2 = s2 + o;
-            const float2 *w = sw + (size_t)xx * WB, *wp = swp + (size_t)xx * WB;
-#pragma unroll 2
-            for (int k = 0; k < n; ++k) term(w[k], wp[k], v0[k * 32], v1[k * 32], v2[k * 32]);
-        } else if (valid) {
-            const float2 *w = t.wf + x, *wp = t.wpf + x;
-            const size_t b = (size_t)s * plane + (size_t)y * d + z;
-            int k = 0;
-            for (; k + kFfBatch <= n; k += kFfBatch) {
-                float2 wx[kFfBatch], wxp[kFfBatch], v0[kFfBatch], v1[kFfBatch], v2[kFfBatch];
+        if (slab) {
+            const float2 *a = (q == 2 ? s1 : s0) + (s - r0) * zw + zz;
+            const float2 *w = (q == 1 ? swp : sw) + (size_t)yy * WB;
+#pragma unroll 4
+            for (int k = k0; k < n; ++k) term(w[k], a[k * zw]);
+        } else {
+            const float2 *w = (q == 1 ? wpf : wf) + y, *A = q == 2 ? A1 : A0;
+            const size_t row = (size_t)xp * S1 + s;
+            for (int k = k0; k < n; k += kFfBatch) {
+                float2 wy[kFfBatch], v[kFfBatch];
 #pragma unroll
                 for (int u = 0; u < kFfBatch; ++u) {
-                    const size_t e = b + (size_t)(k + u) * plane;
-                    wx[u] = __ldg(w + (size_t)(k + u) * d);
-                    wxp[u] = __ldg(wp + (size_t)(k + u) * d);
-                    v0[u] = __ldg(B0 + e);
-                    v1[u] = __ldg(B1 + e);
-                    v2[u] = __ldg(B2 + e);
+                    const bool on = k + u < n && t.rowf[row + k + u];
+                    const size_t o = (size_t)(k + u) * d;
+                    wy[u] = on ? __ldg(w + o) : make_float2(0.f, 0.f);
+                    v[u] = on ? __ldg(A + row * d + o + z) : make_float2(0.f, 0.f);
                 }
 #pragma unroll
-                for (int u = 0; u < kFfBatch; ++u) term(wx[u], wxp[u], v0[u], v1[u], v2[u]);
-            }
-            for (; k < n; ++k) {
-                const size_t e = b + (size_t)k * plane;
-                term(__ldg(w + (size_t)k * d), __ldg(wp + (size_t)k * d), __ldg(B0 + e), __ldg(B1 + e),
-                     __ldg(B2 + e));
+                for (int u = 0; u < kFfBatch; ++u) term(wy[u], v[u]);
             }
         }
-        const double dt = valid ? (double)dh + (double)dl : 0.0;
-        float v0 = 0.f, v1 = 0.f, v2 = 0.f;
-        if (valid && dt != 0.0) {
-            // VESPER_1_prob_new.py:242-255
-            const double px = (double)xh + (double)xl, py = (double)yh + (double)yl, pz = (double)zh + (double)zl;
-            const double rd = __ddiv_rn(1.0, dt);
-            const double t0 = __dsub_rn(__dmul_rn(px, rd), t.pos[x]);
-            const double t1 = __dsub_rn(__dmul_rn(py, rd), t.pos[d + y]);
-            const double t2 = __dsub_rn(__dmul_rn(pz, rd), t.pos[2 * d + z]);
-            double dv = __dadd_rn(__dmul_rn(t0, t0), __dmul_rn(t1, t1));
-            dv = __dsqrt_rn(__dadd_rn(dv, __dmul_rn(t2, t2)));
-            if (dv == 0.0) dv = 1.0;
-            const double rdv = __ddiv_rn(1.0, dv);
-            v0 = (float)__dmul_rn(t0, rdv);
-            v1 = (float)__dmul_rn(t1, rdv);
-            v2 = (float)__dmul_rn(t2, rdv);
-        }
-        const size_t lin = ((size_t)x * d + y) * d + z;
-        data_out[lin] = dt;
-        if (data_f32) data_f32[lin] = (float)dt;
-        vec_out[3 * lin + 0] = v0;
-        vec_out[3 * lin + 1] = v1;
-        vec_out[3 * lin + 2] = v2;
+        (q == 0 ? B0 : q == 1 ? B1 : B2)[((size_t)xp * d + y) * d + z] = make_float2(bh, bl);
     }
+}
+
+// stage 3 (x) and the finish, four lanes per listed voxel, one for each of its sums
+// D, Px, Py, Pz: the column's sums are read along x between the first and last plane
+// with a non-zero value, kXBatch entries in flight.  Blocks over all voxels, a slab of
+// B0, B1 and B2 in shared memory and 9 of 32 lanes at work took 34 us for 256^3 -> 42^3.
+// With the stages above the whole call went from 233 to 121 us there and from 73 to 59
+// for 128^3 -> 28^3.
+__global__ void __launch_bounds__(128) k_fvf_x(const FvGeom g, const AxisTables t, const float2 *B0, const float2 *B1,
+                                               const float2 *B2, double *data_out, float *data_f32, float *vec_out) {
+    const int i = blockIdx.x * 32 + (threadIdx.x >> 2), q = threadIdx.x & 3, d = g.d, nv = t.count[1];
+    if (blockIdx.x * 32 >= nv) return;
+    const int vi = t.voxels[min(i, nv - 1)], xi = vi / (d * d);
+    const size_t plane = (size_t)d * d;
+    const int s = t.stp[xi], k0 = max(0, t.count[2] - s), n = min(t.len[xi], t.count[3] + 1 - s);
+    const float2 *w = (q == 1 ? t.wpf : t.wf) + xi, *b = (q < 2 ? B0 : q == 2 ? B1 : B2) + (size_t)s * plane + vi % (d * d);
+    float sh = 0.f, sl = 0.f;
+    for (int k = k0; k < n; k += kXBatch) {
+        float2 wx[kXBatch], bv[kXBatch];
+#pragma unroll
+        for (int u = 0; u < kXBatch; ++u) {
+            const int e = min(k + u, n - 1);   // every load is made, so that all are in flight
+            wx[u] = __ldg(w + (size_t)e * d);
+            bv[u] = __ldg(b + (size_t)e * plane);
+            if (k + u >= n) bv[u] = make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < kXBatch; ++u) {
+            float ph, pl;
+            ff_mul(bv[u], wx[u], ph, pl);
+            ff_add(sh, sl, ph, pl);
+        }
+    }
+    // the finish is float64, at 1/64 of the float32 rate: whole warps of voxels
+    __shared__ float2 sums[4][32];
+    sums[q][threadIdx.x >> 2] = make_float2(sh, sl);
+    __syncthreads();
+    const int f = blockIdx.x * 32 + threadIdx.x;
+    if (threadIdx.x >= 32 || f >= nv) return;
+    const int v = t.voxels[f], x = v / (d * d), yz = v - x * d * d, y = yz / d, z = yz - y * d;
+    const float2 sd = sums[0][threadIdx.x], sx = sums[1][threadIdx.x], sy = sums[2][threadIdx.x], sz = sums[3][threadIdx.x];
+    const double dt = (double)sd.x + (double)sd.y;
+    float o0 = 0.f, o1 = 0.f, o2 = 0.f;
+    if (dt != 0.0) {
+        // VESPER_1_prob_new.py:242-255
+        const double px = (double)sx.x + (double)sx.y, py = (double)sy.x + (double)sy.y, pz = (double)sz.x + (double)sz.y;
+        const double rd = __ddiv_rn(1.0, dt);
+        const double t0 = __dsub_rn(__dmul_rn(px, rd), t.pos[x]);
+        const double t1 = __dsub_rn(__dmul_rn(py, rd), t.pos[d + y]);
+        const double t2 = __dsub_rn(__dmul_rn(pz, rd), t.pos[2 * d + z]);
+        double dv = __dadd_rn(__dmul_rn(t0, t0), __dmul_rn(t1, t1));
+        dv = __dsqrt_rn(__dadd_rn(dv, __dmul_rn(t2, t2)));
+        if (dv == 0.0) dv = 1.0;
+        const double rdv = __ddiv_rn(1.0, dv);
+        o0 = (float)__dmul_rn(t0, rdv);
+        o1 = (float)__dmul_rn(t1, rdv);
+        o2 = (float)__dmul_rn(t2, rdv);
+    }
+    data_out[v] = dt;
+    if (data_f32) data_f32[v] = (float)dt;
+    vec_out[3 * (size_t)v + 0] = o0;
+    vec_out[3 * (size_t)v + 1] = o1;
+    vec_out[3 * (size_t)v + 2] = o2;
 }
 
 // smallest band weight of the geometry (|r| <= fmaxd + 1 on each axis)
@@ -630,25 +644,26 @@ static bool fv_float_float(const FvGeom &g) {
     return std::exp(-1.5 * r * r * g.fsiv) >= 0x1p-70;
 }
 
-// chunk size and slab rows of the y and x stages: the chunk's bands cover at
-// most WB + floor((c - 1) dw / sw) + 1 source rows (stp is non-decreasing in
-// the output index and steps by at most floor(dw / sw) + 1); c = 8 outputs per
-// block, fewer while the slab exceeds 100 KB; rmax = 0 (global loads) when even
-// one output's band does not fit
-static void fvf_chunk(const FvGeom &g, int S, int narr, int *c, int *rmax, size_t *bytes) {
-    for (int cc = 8; cc >= 1; cc /= 2) {
+// The y stage's chunk and slab rows: the chunk's bands cover at most WB +
+// floor((c - 1) dw / sw) + 1 source rows (stp is non-decreasing in the output index
+// and steps by at most floor(dw / sw) + 1).  About one column of the chunk per
+// thread, fewer while the slab exceeds 64 KB (three blocks per SM); rmax = 0 (global
+// loads) when even one output's band does not fit.
+static void fvf_chunk(const FvGeom &g, int S, int zw, int *c, int *rmax, size_t *bytes) {
+    const int want = std::min(g.d, (kYThreads + zw - 1) / zw);
+    for (int cc = want; cc >= 1; cc = cc > 1 ? (cc + 1) / 2 : 0) {
         const int r = std::min(S, g.WB + (int)((cc - 1) * g.dw / g.sw) + 2);
-        const size_t b = ((size_t)narr * r * 32 + 2 * (size_t)cc * g.WB) * sizeof(float2);
-        if (b <= 100 * 1024 || (cc == 1 && b <= 200 * 1024)) {
+        const size_t b = ((size_t)2 * r * zw + 2 * (size_t)cc * g.WB) * sizeof(float2) + (size_t)cc * zw * sizeof(short);
+        if (b <= 64 * 1024 || (cc == 1 && b <= 200 * 1024)) {
             *c = cc;
             *rmax = r;
             *bytes = b;
             return;
         }
     }
-    *c = 8;
+    *c = 1;
     *rmax = 0;
-    *bytes = 0;
+    *bytes = 2 * (size_t)g.WB * sizeof(float2) + (size_t)zw * sizeof(short);
 }
 
 static void fv_geom(int sx, int sy, int sz, double src_width, const double *src_orig, int dim, double dest_width,
@@ -684,9 +699,13 @@ static size_t fv_workspace(const FvGeom &g, AxisTables *t, double **A0, double *
     t->wp = cv.take<double>(3 * (size_t)g.WB * d);
     t->wf = cv.take<float2>(3 * (size_t)g.WB * d);
     t->wpf = cv.take<float2>(3 * (size_t)g.WB * d);
-    t->plane = cv.take<int>((size_t)g.S[0]);
+    t->rlo = cv.take<int>((size_t)g.S[0]);
+    t->rhi = cv.take<int>((size_t)g.S[0]);
     t->list = cv.take<int>((size_t)g.S[0] * g.S[1]);
-    t->nlist = cv.take<int>(1);
+    t->rowf = cv.take<unsigned char>((size_t)g.S[0] * g.S[1]);
+    t->need = cv.take<unsigned char>((size_t)d * d);
+    t->voxels = cv.take<int>((size_t)d * d * d);
+    t->count = cv.take<int>(4);
     // the partial sums: float64, or float-float pairs of the same 8 bytes
     const size_t rows = (size_t)g.S[0] * g.S[1];
     *A0 = cv.take<double>(rows * d);
@@ -739,36 +758,41 @@ extern "C" int vesper_fastvec(const float *src, int sx, int sy, int sz, double s
     VG_CHECK_LAUNCH("k_fv_tables");
     const size_t nrows = (size_t)sx * sy;
     if (fv_float_float(g)) {
-        const size_t srows = (size_t)(kZRows + 1) * sz * sizeof(float);
-        const size_t sweights = 2 * (size_t)g.WB * dim * sizeof(float2);
-        const bool zsw = srows + sweights <= 100 * 1024;   // the z weights staged in shared memory
-        const size_t s1 = srows + (zsw ? sweights : 0);
-        if (s1 > 200 * 1024) return fail(VESPER_ERR_UNSUPPORTED, "vesper_fastvec: source rows too long (%d)", sz);
+        if ((size_t)17 * sz * sizeof(float) > 200 * 1024)
+            return fail(VESPER_ERR_UNSUPPORTED, "vesper_fastvec: source rows too long (%d)", sz);
         float2 *a0 = reinterpret_cast<float2 *>(A0), *a1 = reinterpret_cast<float2 *>(A1);
         float2 *b0 = reinterpret_cast<float2 *>(B0), *b1 = reinterpret_cast<float2 *>(B1),
                *b2 = reinterpret_cast<float2 *>(B2);
-        k_fvf_rows<<<(unsigned)std::min<size_t>((nrows + 7) / 8, 4096), 256, 0, st>>>(src, g, t, a0, a1);
-        VG_CHECK_LAUNCH("k_fvf_rows");
-        const unsigned zb = (unsigned)((nrows + kZRows - 1) / kZRows);
+        const unsigned row_blocks = (unsigned)std::min<size_t>((nrows + 63) / 64, 1 << 14);
+        const unsigned vox_blocks = (unsigned)(((size_t)dim * dim * dim + 255) / 256);
+        if (sz % 4 == 0 && ((uintptr_t)src & 15) == 0)
+            k_fvf_scan<true><<<row_blocks + vox_blocks, 256, 0, st>>>(src, g, t, (int)row_blocks, data_out, data_f32, vec_out);
+        else
+            k_fvf_scan<false><<<row_blocks + vox_blocks, 256, 0, st>>>(src, g, t, (int)row_blocks, data_out, data_f32, vec_out);
+        VG_CHECK_LAUNCH("k_fvf_scan");
+        int rows = kZRows;
+        while (rows > 1 && fvf_z_rows_smem(sz, rows) > 64 * 1024) rows /= 2;
+        const size_t srows = fvf_z_rows_smem(sz, rows), sweights = 2 * (size_t)g.WB * dim * sizeof(float2);
+        const bool zsw = srows + sweights <= 112 * 1024;   // the z weights staged in shared memory, two blocks per SM
+        const size_t s1 = srows + (zsw ? sweights : 0);
+        const unsigned zb = (unsigned)((nrows + rows - 1) / rows);
         if (zsw) {
             allow_smem(k_fvf_z<true>, s1);
-            k_fvf_z<true><<<zb, 256, s1, st>>>(src, g, t, a0, a1);
+            k_fvf_z<true><<<zb, kZThreads, s1, st>>>(src, g, t, rows, a0, a1);
         } else {
             allow_smem(k_fvf_z<false>, s1);
-            k_fvf_z<false><<<zb, 256, s1, st>>>(src, g, t, a0, a1);
+            k_fvf_z<false><<<zb, kZThreads, s1, st>>>(src, g, t, rows, a0, a1);
         }
         VG_CHECK_LAUNCH("k_fvf_z");
-        const unsigned zt = (unsigned)((dim + 31) / 32);
-        int yc, ry, xc, rx;
-        size_t sy2, sx3;
-        fvf_chunk(g, sy, 2, &yc, &ry, &sy2);
-        fvf_chunk(g, sx, 3, &xc, &rx, &sx3);
+        const int nt = (dim + 31) / 32, zw = (dim + nt - 1) / nt;
+        int yc, ry;
+        size_t sy2;
+        fvf_chunk(g, sy, zw, &yc, &ry, &sy2);
         allow_smem(k_fvf_y, sy2);
-        k_fvf_y<<<dim3(zt, sx, (unsigned)((dim + yc - 1) / yc)), 256, sy2, st>>>(g, t, yc, ry, a0, a1, b0, b1, b2);
+        k_fvf_y<<<dim3(nt, sx, (unsigned)((dim + yc - 1) / yc)), kYThreads, sy2, st>>>(g, t, zw, yc, ry, a0, a1, b0, b1, b2);
         VG_CHECK_LAUNCH("k_fvf_y");
-        allow_smem(k_fvf_x, sx3);
-        k_fvf_x<<<dim3(zt, dim, (unsigned)((dim + xc - 1) / xc)), 256, sx3, st>>>(src, g, t, xc, rx, b0, b1, b2,
-                                                                                  data_out, data_f32, vec_out);
+        k_fvf_x<<<(unsigned)(((size_t)dim * dim * dim + 31) / 32), 128, 0, st>>>(g, t, b0, b1, b2, data_out, data_f32,
+                                                                                   vec_out);
         VG_CHECK_LAUNCH("k_fvf_x");
         return VESPER_OK;
     }
