@@ -17,14 +17,17 @@
 // steps in the opposite order.
 //
 // What bounds them (GB300, mode V, microseconds per rotation A / B / C, against
-// the kernels they replace): side 75 3.14 / 1.52 / 0.99 (one block-wide step after
-// another, general gather in line: 5.41 / 1.74 / 1.04), side 48 0.89 / 0.67 / 0.30
-// (radix stages 2.26 / 1.60 / 1.06), side 80 3.73 / 2.4 / 1.14 (11.9 / 7.4 / 3.1),
-// prob mode at side 64 6.4 / 3.4 / 2.7 (18.0 / 5.4 / 2.7).  A is bound by issue
+// the kernels they replace): side 75 3.14 / 1.52 / 0.87 (one block-wide step after
+// another, general gather in line: 5.41 / 1.74 / 1.04), side 48 0.82 / 0.66 / 0.29
+// (radix stages 2.26 / 1.60 / 1.06), side 80 3.48 / 2.4 / 1.12 (11.9 / 7.4 / 3.1),
+// prob mode at side 64 4.0 / 2.6 / 1.16 (18.0 / 5.4 / 2.7).  A is bound by issue
 // slots and shared-memory wavefronts together (56 % and 58 % at 15 warps per SM;
 // one warp per tile gives 30): strides without bank conflicts took side 75 from
 // 4.17 to 3.93, one warp per tile within 64 registers to 3.48, and the middle
-// voxels of odd sides, loaded together and shared out over the CTA, to 3.14.  B is
+// voxels of odd sides, loaded together and shared out over the CTA, to 3.14; prob mode
+// at side 64 4.51 -> 3.97 with lines and columns that do not meet in a bank.  C is bound
+// by issue slots (75 %): one 32-bit comparison per voxel instead of a 64-bit key took
+// side 75 from 0.98 to 0.87.  B is
 // bound by the S and T it reads: T from L2 once per 8 rotations instead of once
 // each took side 75 from 1.74 to 1.52.
 #pragma once
@@ -40,7 +43,8 @@ namespace vg {
 // apart, so lanes that run over 4 lines and then over 4 consecutive elements cover
 // all 16; between the steps element (k1, j2) of a line sits at P2 k1 + j2 with P2
 // odd, so that runs over k1 do the same; CS = N2 mod 4 continues the pattern
-// from one channel to the next.
+// from one channel to the next (2 where N2 is a multiple of 4: runs over 8 lines of
+// two channels).
 constexpr int up_to_mod(int n, int mod, int rem) { return n + ((rem - n) % mod + mod) % mod; }
 // SPLIT: a line's elements lie half in its first row's storage, half in its second's.
 template <int N1, int N2, bool SPLIT = false>
@@ -50,13 +54,34 @@ struct TGeom {
     static constexpr int kHalf = SPLIT ? (N1 + 1) / 2 * P2 : (N1 * P2 + 1) / 2;
     static constexpr int RS = up_to_mod(H > kHalf ? H : kHalf, 4, 2);   // row stride
     static constexpr int LS = 2 * RS;          // packed line p lives in rows 2p and 2p + 1
-    static constexpr int CS = up_to_mod(NP * LS, 4, N2 % 4);   // channel stride
+    static constexpr int CS = up_to_mod(NP * LS, 4, N2 % 4 ? N2 % 4 : 2);   // channel stride
     static constexpr int TP = (NP + 3) / 4;    // gather tiles of 4 lines
     // where element z = j2 + N2 j1 of a line waits for step 1
     static __device__ __forceinline__ int pos(int z) { return P2 == N2 ? z : z / N2 * P2 + z % N2; }
 };
 
+// Column kz and row of item t of a step along y in shared memory: a half warp stays in one
+// row as long as that leaves no lane idle (runs over whole rows of H put two rows into
+// most half warps, whose banks overlap), the columns past the last 16 of each row follow.
+template <int H> __device__ __forceinline__ void column_item(int t, int rows, int &kz, int &row) {
+    constexpr int HM = H / 16 * 16, HR = H - HM;
+    const int u = t - rows * HM;
+    if (HM && u < 0) {
+        row = t / (HM ? HM : 1);
+        kz = t - row * HM;
+    } else {
+        row = u / (HR ? HR : 1);
+        kz = HM + u - row * HR;
+    }
+}
+
 // ---- pass A -------------------------------------------------------------------
+// Lines per round of the second z step: as many as the warp's lanes hold, whole groups
+// of 4 (which fall in different banks) where that costs no round.
+__host__ __device__ constexpr int lines_per_round(int items, int lines) {
+    const int most = 32 / items < lines ? 32 / items : lines, four = most / 4 * 4;
+    return four && (lines + four - 1) / four == (lines + most - 1) / most ? four : most;
+}
 template <int SRC, int N1, int N2>
 __host__ __device__ constexpr size_t smem_ta() {
     using G = TGeom<N1, N2>;
@@ -104,10 +129,12 @@ __device__ __forceinline__ void tpass_a(const PassA2 &a, int c0) {
             }
         }
         __syncwarp();
-        // z step 2 and unpack into the line's own two rows: items (line, q), q
-        // in [0, N1/2], whole lines per round, read before they are written
-        constexpr int NQ = N1 / 2 + 1, LPR = 32 / NQ;
-        const int lq = lane % LPR, q = lane / LPR, q2 = (N1 - q) % N1;   // line fastest
+        // z step 2 and unpack into the line's own two rows: items (line, q) of k1 = q and its
+        // mirror N1 - q (q = 0: 0 and, N1 even, N1 / 2, which mirror themselves), whole
+        // lines per round, read before they are written
+        constexpr bool EV = N1 % 2 == 0;
+        constexpr int NQ = (N1 + 1) / 2, LPR = lines_per_round(NQ, NCH * 4);
+        const int lq = lane % LPR, q = lane / LPR, q2 = q ? N1 - q : EV ? N1 / 2 : 0;   // line fastest
 #pragma unroll 1
         for (int l0 = 0; l0 < NCH * 4; l0 += LPR) {
             const int l = l0 + lq, p = pt * 4 + (l & 3), c = l >> 2;
@@ -135,9 +162,9 @@ __device__ __forceinline__ void tpass_a(const PassA2 &a, int c0) {
                         row1[k] = B;
                     }
                     const int kb = q2 + N1 * k2;
-                    if (q != 0 && q2 != q && kb < H) {
+                    if ((EV || q != 0) && kb < H) {
                         float2 A, B;
-                        unpack_pair(w2[k2], u[N2 - 1 - k2], A, B);
+                        unpack_pair(w2[k2], (q == 0) ? w2[N2 - 1 - k2] : u[N2 - 1 - k2], A, B);
                         row0[kb] = A;
                         row1[kb] = B;
                     }
@@ -148,7 +175,9 @@ __device__ __forceinline__ void tpass_a(const PassA2 &a, int c0) {
     __syncthreads();
     // y step 1, in place: items (c, j2, kz), kz fastest
     for (int t = threadIdx.x; t < NCH * N2 * H; t += NW * 32) {
-        const int kz = t % H, cj = t / H, j2 = cj % N2, c = cj / N2;
+        int kz, cj;
+        column_item<H>(t, NCH * N2, kz, cj);
+        const int j2 = cj % N2, c = cj / N2;
         float2 *col = buf + c * CS + j2 * RS + kz;
         float2 v[N1];
 #pragma unroll
@@ -359,7 +388,9 @@ __global__ void __launch_bounds__(tc_warps<N1, N2>() * 32) k_tpass_c(const PassC
         }
         __syncthreads();
         for (int t = threadIdx.x; t < NGRP * N1 * H; t += NW * 32) {
-            const int kz = t % H, gk = t / H, k1 = gk % N1, g = gk / N1;
+            int kz, gk;
+            column_item<H>(t, NGRP * N1, kz, gk);
+            const int k1 = gk % N1, g = gk / N1;
             float2 *col = buf + g * CS + N2 * k1 * RS + kz;
             float2 u[N2];
 #pragma unroll
@@ -385,7 +416,9 @@ __global__ void __launch_bounds__(tc_warps<N1, N2>() * 32) k_tpass_c(const PassC
         __syncthreads();
         // inverse y step 1, in place: items (g, j2, kz) -> rows y = j2 + N2 j1
         for (int t = threadIdx.x; t < NGRP * N2 * H; t += NW * 32) {
-            const int kz = t % H, gj = t / H, j2 = gj % N2, g = gj / N2;
+            int kz, gj;
+            column_item<H>(t, NGRP * N2, kz, gj);
+            const int j2 = gj % N2, g = gj / N2;
             float2 *col = buf + g * CS + j2 * RS + kz;
             float2 v[N1];
 #pragma unroll
@@ -398,17 +431,36 @@ __global__ void __launch_bounds__(tc_warps<N1, N2>() * 32) k_tpass_c(const PassC
     }
     const int p0 = warp * PL, pn = min(PL, NP - p0);   // pn <= 0: no line left for this warp
     unsigned long long best[3] = {0ull, 0ull, 0ull};
-    // scores s0 (and s1) of voxel (y, z)
-    auto score = [&](float s0, float s1, int y, int z) {
-        const uint32_t lin = (uint32_t)((x * D + y) * D + z);
-        best[0] = max(best[0], make_key(s0, lin));
-        if (SC >= 2) best[1] = max(best[1], make_key(s1, lin));
+    // Best of one item's voxels, which come in ascending index order: the first of the
+    // greatest scores, as offsets from the item's first voxel (half the instructions of
+    // a 64-bit key per voxel); merged as keys once per item.
+    // float_order as a signed value: the sum makes -0 a +0.
+    int top[SC], at[SC];
+    auto take = [&](int s, float v, int off) {
+        const int i = __float_as_int(__fadd_rn(v, 0.f)), o = i ^ (i >> 31 & 0x7fffffff);
+        if (o > top[s]) {
+            top[s] = o;
+            at[s] = off;
+        }
+    };
+    auto score = [&](float s0, float s1, int off) {
+        take(0, s0, off);
+        if (SC >= 2) take(SC >= 2 ? 1 : 0, s1, off);
         if (SC == 3) {
             const float sv = __fdiv_rn(__fsub_rn(s0, a.mix.vave), a.mix.vstd);
             const float sp = __fdiv_rn(__fsub_rn(s1, a.mix.pave), a.mix.pstd);
-            best[2] = max(best[2], make_key(__fadd_rn(__fmul_rn(a.mix.one_minus_alpha, sv),
-                                                      __fmul_rn(a.mix.alpha, sp)), lin));
+            take(SC == 3 ? 2 : 0, __fadd_rn(__fmul_rn(a.mix.one_minus_alpha, sv), __fmul_rn(a.mix.alpha, sp)), off);
         }
+    };
+    auto begin = [&]() {
+#pragma unroll
+        for (int s = 0; s < SC; ++s) top[s] = (int)0x80000000, at[s] = 0;
+    };
+    auto merge = [&](int y, int z) {
+#pragma unroll
+        for (int s = 0; s < SC; ++s)
+            best[s] = max(best[s], (unsigned long long)((uint32_t)top[s] ^ 0x80000000u) << 32 |
+                                       (0xffffffffu - (uint32_t)((x * D + y) * D + z + at[s])));
     };
     if constexpr (!PFA) {
         // z in the forward's order, each line in its own two rows' storage (elements
@@ -458,23 +510,25 @@ __global__ void __launch_bounds__(tc_warps<N1, N2>() * 32) k_tpass_c(const PassC
                 for (int j2 = 0; j2 < N2; ++j2) u1[j2] = buf[CS + at + j2];
                 rdft_plan<N2, true, N1>(u1, twn);
             }
+            begin();
 #pragma unroll
-            for (int k2 = 0; k2 < N2; ++k2) {
-                const int z = k1 + N1 * k2;
-                score(u0[k2].x, NGRP == 2 ? u1[k2].x : 0.f, 2 * p, z);
-                if (hb) score(u0[k2].y, NGRP == 2 ? u1[k2].y : 0.f, 2 * p + 1, z);
-            }
+            for (int k2 = 0; k2 < N2; ++k2) score(u0[k2].x, NGRP == 2 ? u1[k2].x : 0.f, N1 * k2);
+            if (hb)
+#pragma unroll
+                for (int k2 = 0; k2 < N2; ++k2) score(u0[k2].y, NGRP == 2 ? u1[k2].y : 0.f, D + N1 * k2);
+            merge(2 * p, k1);
         }
     } else {
         // z: rows (2p, 2p + 1) as one full line (Hermitian completion, DC and Nyquist
         // imaginary parts dropped), inverse step 2 in the rows' own storage: items
         // (g, line, k1), whole lines per round, read before they are written
         constexpr int LPR = 32 / N1;
-        const int lk1 = lane % N1, lq = lane / N1;
+        constexpr bool LF = LPR % 4 == 0;   // line fastest: 4 lines fall in different banks
+        const int lk1 = LF ? lane / LPR : lane % N1, lq = LF ? lane % LPR : lane / N1;
 #pragma unroll 1
         for (int l0 = 0; l0 < NGRP * pn; l0 += LPR) {
             const int l = l0 + lq, g = NGRP == 2 ? l / max(pn, 1) : 0, p = p0 + l - g * pn;
-            const bool on = lq < LPR && l < NGRP * pn;
+            const bool on = lq < LPR && lk1 < N1 && l < NGRP * pn;
             float2 *line = buf + g * CS + p * LS;
             const bool hb = 2 * p + 1 < D;
             float2 u[N2];
@@ -513,16 +567,13 @@ __global__ void __launch_bounds__(tc_warps<N1, N2>() * 32) k_tpass_c(const PassC
                 for (int k1 = 0; k1 < N1; ++k1) v1[k1] = l0[CS + P2 * k1];
                 rdft<N1, true>(v1);
             }
+            begin();
 #pragma unroll
-            for (int j1 = 0; j1 < N1; ++j1) {
-                const int z = j2 + N2 * j1;
+            for (int j1 = 0; j1 < N1; ++j1) score(v0[j1].x, NGRP == 2 ? v1[j1].x : 0.f, N2 * j1);
+            if (2 * p + 1 < D)
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const int y = 2 * p + half;
-                    if (y >= D) break;
-                    score(half ? v0[j1].y : v0[j1].x, NGRP == 2 ? (half ? v1[j1].y : v1[j1].x) : 0.f, y, z);
-                }
-            }
+                for (int j1 = 0; j1 < N1; ++j1) score(v0[j1].y, NGRP == 2 ? v1[j1].y : 0.f, D + N2 * j1);
+            merge(2 * p, j2);
         }
     }
 #pragma unroll
