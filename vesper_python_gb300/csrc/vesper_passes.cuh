@@ -60,6 +60,9 @@ __device__ __forceinline__ void init_head(const FftPlan &P, const Head &h) {
 }
 
 // ---- pass A -------------------------------------------------------------------
+// Sides up to here take whole lines in registers, larger ones two steps (register passes).
+constexpr int kLineSide = 32;
+
 struct PassA2 {
     Src src;
     const float *rotmats;
@@ -69,6 +72,7 @@ struct PassA2 {
     unsigned long long *keys;     // [nrot][nscore]
     const double *rd;             // Laplacian mode: [batch][d^3] rotated density, or null
     const float *plain;           // Laplacian mode, register passes: [batch][d^3] filtered density
+    const unsigned *reach;        // two-step register passes: voxel_reach of q4 and of p4
 };
 
 // Pass-A sample of rotation b of the batch: the Laplacian mode reads the

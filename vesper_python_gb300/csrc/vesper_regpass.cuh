@@ -67,7 +67,7 @@ __device__ __forceinline__ void rpass_a_line(const PassA2 &a, int c0) {
     float F[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) F[i] = __ldg(a.rotmats + (size_t)r * 9 + i);
-    gather_planes<SRC, D, LS, PS, T / 32>(a, F, b, x0, pn, buf, [](int z) { return z; });
+    gather_planes<SRC, D, LS, PS, T / 32, false>(a, F, b, x0, pn, buf, [](int z) { return z; });
     __syncthreads();
     // z: one packed line per thread; DFT and unpack into rows 2p (offset 0)
     // and 2p + 1 (offset Hp) of the line's own storage
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kLineBThreads) k_rpass_b_line_prob(const PassB
 // mode V: side 30 0.065 (2 planes; 0.092 for the two-step kernel with block
 // barriers between its steps), side 28 0.057 (4), side 32 0.080 (4; 0.104 with 7
 // planes on 128 threads, although those leave fewer idle).
-template <int D> __host__ __device__ constexpr bool line_c_used() { return D <= 32; }
+template <int D> __host__ __device__ constexpr bool line_c_used() { return D <= kLineSide; }
 template <int D> __host__ __device__ constexpr LineShape line_c_shape() {
     constexpr int NP = (D + 1) / 2, H = D / 2 + 1;
     LineShape best{1, 32};
@@ -340,7 +340,7 @@ inline int tb_rotations(int nbx, int nb) {
 template <int N1, int N2, bool PFA, int KINDS>
 struct RegSide {
     static constexpr int D = N1 * N2, H = D / 2 + 1;
-    static constexpr bool kLine = D <= 32;
+    static constexpr bool kLine = D <= kLineSide;
     static_assert(PFA || kLine || plan_last<D>() == N2, "the second step is the plan's last stage");
 
     template <int SRC>

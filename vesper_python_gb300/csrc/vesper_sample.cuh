@@ -27,10 +27,27 @@ __device__ __forceinline__ float query_value(double v, double ave) {
     return 0.f;
 }
 
+// Reach of the voxels with a value: the greatest squared distance of a corner of such a
+// voxel from the grid's centre, as the bits of a float (0: no voxel).  No rotated voxel
+// further out has a source with a value.
+__device__ __forceinline__ void voxel_reach(size_t i, int d, bool on, float &r2) {
+    if (!on) return;
+    const int q = (int)(i / d), z = (int)(i - (size_t)q * d), x = q / d, y = q - x * d;
+    const float h = 0.5f * (float)d, fx = (float)x - h, fy = (float)y - h, fz = (float)z - h;
+    const float tx = fmaxf(-fx, fx + 1.f), ty = fmaxf(-fy, fy + 1.f), tz = fmaxf(-fz, fz + 1.f);
+    r2 = fmaxf(r2, tx * tx + ty * ty + tz * tz);
+}
+__device__ __forceinline__ void store_reach(float r2, unsigned *reach) {   // whole warps
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(r2));
+    if (m && (threadIdx.x & 31) == 0) atomicMax(reach, m);
+}
+
+// reach (or null): of the vectors or values, and of the probabilities
 template <int MODE>
 __global__ void k_pack(const double *data, const float *vec, const float *probs, int d, double ave, float4 *q4,
-                       float4 *p4) {
+                       float4 *p4, unsigned *reach) {
     const size_t n = (size_t)d * d * d;
+    float r2 = 0.f, rp = 0.f;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double v = data[i];
         const float m = v != 0.0 ? 1.f : 0.f;
@@ -42,18 +59,30 @@ __global__ void k_pack(const double *data, const float *vec, const float *probs,
             o = make_float4(query_value<MODE>(v, ave), 0.f, 0.f, m);
         }
         q4[i] = o;
-        if (MODE == VESPER_MODE_PROB) p4[i] = make_float4(probs[i], probs[n + i], probs[2 * n + i], probs[3 * n + i]);
+        if (reach) voxel_reach(i, d, m != 0.f, r2);
+        if (MODE == VESPER_MODE_PROB) {
+            const float4 p = make_float4(probs[i], probs[n + i], probs[2 * n + i], probs[3 * n + i]);
+            p4[i] = p;
+            if (reach) voxel_reach(i, d, p.x != 0.f || p.y != 0.f || p.z != 0.f || p.w != 0.f, rp);
+        }
     }
+    if (reach) store_reach(r2, reach);
+    if (MODE == VESPER_MODE_PROB && reach) store_reach(rp, reach + 1);
 }
 
 // The value of the scalar modes alone (4 bytes a voxel: a gather's cache lines
 // hold four times as many), for the register passes; it is zero wherever the
 // density is.
 template <int MODE>
-__global__ void k_pack_value(const double *data, int d, double ave, float *q1) {
+__global__ void k_pack_value(const double *data, int d, double ave, float *q1, unsigned *reach) {
     const size_t n = (size_t)d * d * d;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        q1[i] = query_value<MODE>(data[i], ave);
+    float r2 = 0.f;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const double v = data[i];
+        q1[i] = query_value<MODE>(v, ave);
+        if (reach) voxel_reach(i, d, v != 0.0, r2);
+    }
+    if (reach) store_reach(r2, reach);
 }
 
 // ---- gather -----------------------------------------------------------------

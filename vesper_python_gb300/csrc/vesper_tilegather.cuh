@@ -106,8 +106,10 @@ __device__ __forceinline__ void store_pair(float2 *at, int p, int z, float v0, f
 // share cache lines in all three directions.  A voxel with one candidate row per
 // axis is one load (its position's x and y terms are kept per row); the voxels
 // of an odd side's middle index (3 D^2 of D^3) are left to gather_planes.
-template <int SRC, int D, int LS, int CS, class Pos>
-__device__ __forceinline__ void gather_tile(const PassA2 &a, const float (&F)[9], int b, int x, int pt, float2 *buf,
+// REACH: only the z steps that come within the query's reach are looked at; returns
+// whether no voxel of the tile does (nothing is stored then).
+template <int SRC, int D, int LS, int CS, bool REACH, class Pos>
+__device__ __forceinline__ bool gather_tile(const PassA2 &a, const float (&F)[9], int b, int x, int pt, float2 *buf,
                                             Pos pos) {
     constexpr int NCH = src_nch<SRC>(), NP = (D + 1) / 2, TZ = (D + 7) / 8;
     constexpr int GI = TZ % 3 == 0 ? 3 : TZ % 2 == 0 ? 2 : TZ % 5 == 0 ? 5 : 2;   // z steps whose loads are in flight together
@@ -122,7 +124,7 @@ __device__ __forceinline__ void gather_tile(const PassA2 &a, const float (&F)[9]
             const int z = t * 8 + zl;
             if (pon && z < D) line[pos(z)] = make_float2(__ldg(src + z), 2 * p + 1 < D ? __ldg(src + D + z) : 0.f);
         }
-        return;
+        return false;
     } else {
         constexpr float hc = 0.5f * (float)D, df = (float)D;
         const bool xon = has_cand<D>(x);
@@ -137,8 +139,43 @@ __device__ __forceinline__ void gather_tile(const PassA2 &a, const float (&F)[9]
 #pragma unroll
             for (int i = 0; i < 3; ++i) base[h][i] = __fmaf_rn(hy, F[i * 3 + 1], __fmul_rn(hx, F[i * 3]));
         }
+        int z0 = 0, z1 = D - 1;   // steps outside hold no value
+        if constexpr (REACH) {
+            // |base + hz c|^2 <= reach, c the matrix's third column: an interval of hz per row.
+            // Wide by a voxel for the rounding and one for the first candidates' offset, and
+            // only for columns of about unit length, where neither can be more.
+            const float r2 = __uint_as_float(__ldg(a.reach + (SRC == kSrcProb))) + 1.f;
+            const float cc = F[2] * F[2] + F[5] * F[5] + F[8] * F[8];
+            if (cc > 0.5f && cc < 2.f) {
+                z0 = D, z1 = -1;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float bc = base[h][0] * F[2] + base[h][1] * F[5] + base[h][2] * F[8];
+                    const float bb = base[h][0] * base[h][0] + base[h][1] * base[h][1] + base[h][2] * base[h][2] - r2;
+                    const float disc = bc * bc - cc * bb;
+                    if (!on[h] || disc < 0.f) continue;
+                    const float sq = sqrtf(disc), lo = (-bc - sq) / cc + hc, hi = (-bc + sq) / cc + hc;
+                    z0 = min(z0, (int)fminf(fmaxf(lo, 0.f), df) - 3);
+                    z1 = max(z1, (int)fminf(fmaxf(hi, -4.f), df) + 2);
+                }
+                z0 = __reduce_min_sync(0xffffffffu, z0);
+                z1 = __reduce_max_sync(0xffffffffu, z1);
+                // the tile of an odd side's middle row has voxels of another row's position
+                if (z0 > z1 && ((D & 1) == 0 || pt != (D - 1) / 16)) return true;
+            }
+        }
 #pragma unroll 1
         for (int t0 = 0; t0 < TZ; t0 += GI) {
+            if (REACH && (t0 * 8 > z1 || (t0 + GI) * 8 <= z0)) {
+#pragma unroll
+                for (int g = 0; g < GI; ++g) {
+                    const int z = (t0 + g) * 8 + zl;
+                    if (pon && z < D)
+#pragma unroll
+                        for (int c = 0; c < NCH; ++c) store_pair<D>(line + c * CS + pos(z), p, z, 0.f, 0.f);
+                }
+                continue;
+            }
             int src[GI][2];
 #pragma unroll
             for (int g = 0; g < GI; ++g) {
@@ -197,14 +234,16 @@ __device__ __forceinline__ void gather_tile(const PassA2 &a, const float (&F)[9]
             }
         }
     }
+    return false;
 }
 
 // Gather of pn planes from x0 by a CTA of NW warps, each into tiles of its own (plane
 // stride: the source's channels times CS); on an odd side the voxels of the middle
 // index are shared out over the whole CTA first (2 D - 1 of a plane, or all of the
 // middle plane and the row that its last line lacks).  Ready after a block barrier.
-template <int SRC, int D, int LS, int CS, int NW, class Pos>
-__device__ __forceinline__ void gather_planes(const PassA2 &a, const float (&F)[9], int b, int x0, int pn, float2 *buf,
+// REACH (a tile per warp): whether the warp's tile holds no value and is unwritten.
+template <int SRC, int D, int LS, int CS, int NW, bool REACH, class Pos>
+__device__ __forceinline__ bool gather_planes(const PassA2 &a, const float (&F)[9], int b, int x0, int pn, float2 *buf,
                                               Pos pos) {
     constexpr int NCH = src_nch<SRC>(), TP = ((D + 1) / 2 + 3) / 4;
     if constexpr (SRC == kSrcVec) {
@@ -215,7 +254,7 @@ __device__ __forceinline__ void gather_planes(const PassA2 &a, const float (&F)[
         for (int i = 0; i < 9; ++i) finite = finite && fabsf(F[i]) <= 3.4028234e38f;
         if (!finite) {
             for (int e = threadIdx.x; e < pn * 3 * CS; e += NW * 32) buf[e] = make_float2(0.f, 0.f);
-            return;
+            return false;
         }
     }
     if constexpr ((D & 1) != 0 && SRC != kSrcPlain) {
@@ -240,11 +279,13 @@ __device__ __forceinline__ void gather_planes(const PassA2 &a, const float (&F)[
                 put(M - x0, e / D, e % D, o);
             }
     }
+    bool empty = false;
     for (int pt = threadIdx.x >> 5; pt < pn * TP; pt += NW) {
         const int pl = pt / TP, x = x0 + pl;
         if ((D & 1) != 0 && SRC != kSrcPlain && x == (D - 1) / 2) continue;
-        gather_tile<SRC, D, LS, CS>(a, F, b, x, pt - pl * TP, buf + pl * NCH * CS, pos);
+        empty = gather_tile<SRC, D, LS, CS, REACH>(a, F, b, x, pt - pl * TP, buf + pl * NCH * CS, pos);
     }
+    return empty;
 }
 
 }  // namespace vg

@@ -17,15 +17,18 @@
 // steps in the opposite order.
 //
 // What bounds them (GB300, mode V, microseconds per rotation A / B / C, against
-// the kernels they replace): side 75 3.14 / 1.52 / 0.87 (one block-wide step after
-// another, general gather in line: 5.41 / 1.74 / 1.04), side 48 0.82 / 0.66 / 0.29
-// (radix stages 2.26 / 1.60 / 1.06), side 80 3.48 / 2.4 / 1.12 (11.9 / 7.4 / 3.1),
-// prob mode at side 64 4.0 / 2.6 / 1.16 (18.0 / 5.4 / 2.7).  A is bound by issue
+// the kernels they replace): side 75 2.50 / 1.52 / 0.87 (one block-wide step after
+// another, general gather in line: 5.41 / 1.74 / 1.04), side 48 0.67 / 0.66 / 0.29
+// (radix stages 2.26 / 1.60 / 1.06), side 80 2.72 / 2.4 / 1.12 (11.9 / 7.4 / 3.1),
+// prob mode at side 64 3.3 / 2.6 / 1.16 (18.0 / 5.4 / 2.7).  A is bound by issue
 // slots and shared-memory wavefronts together (56 % and 58 % at 15 warps per SM;
 // one warp per tile gives 30): strides without bank conflicts took side 75 from
 // 4.17 to 3.93, one warp per tile within 64 registers to 3.48, and the middle
 // voxels of odd sides, loaded together and shared out over the CTA, to 3.14; prob mode
-// at side 64 4.51 -> 3.97 with lines and columns that do not meet in a bank.  C is bound
+// at side 64 4.51 -> 3.97 with lines and columns that do not meet in a bank.  A query
+// fills a ball of its grid, and the rotated one a ball too: leaving out the z steps,
+// lines and planes outside it took side 75 from 3.14 to 2.50 and prob mode at side 64
+// from 3.97 to 3.30 (a ball of 0.42 of the side).  C is bound
 // by issue slots (75 %): one 32-bit comparison per voxel instead of a 64-bit key took
 // side 75 from 0.98 to 0.87.  B is
 // bound by the S and T it reads: T from L2 once per 8 rotations instead of once
@@ -112,9 +115,16 @@ __device__ __forceinline__ void tpass_a(const PassA2 &a, int c0) {
     float F[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) F[i] = __ldg(a.rotmats + (size_t)r * 9 + i);
-    gather_planes<SRC, D, LS, CS, NW>(a, F, b, x, 1, buf, [](int z) { return G::pos(z); });
+    static_assert(NW == G::TP, "one tile per warp");
+    const bool empty = gather_planes<SRC, D, LS, CS, NW, true>(a, F, b, x, 1, buf, [](int z) { return G::pos(z); });
     __syncthreads();
-    for (int pt = warp; pt < G::TP; pt += NW) {
+    const int pt = warp;
+    if (empty) {   // zeros transform to zeros
+        for (int l = 0; l < 4 && pt * 4 + l < NP; ++l)
+#pragma unroll
+            for (int c = 0; c < NCH; ++c)
+                for (int k = lane; k < LS; k += 32) buf[c * CS + (pt * 4 + l) * LS + k] = make_float2(0.f, 0.f);
+    } else {
         // z step 1, in place: items (c, j2, line), line fastest
         for (int it = lane; it < NCH * 4 * N2; it += 32) {
             const int p = pt * 4 + (it & 3), j2 = (it >> 2) % N2, c = (it >> 2) / N2;
@@ -172,7 +182,12 @@ __device__ __forceinline__ void tpass_a(const PassA2 &a, int c0) {
             }
         }
     }
-    __syncthreads();
+    float2 *out = a.S + (((size_t)b * a.nch + c0) * D + x) * (size_t)(D * H);
+    if (!__syncthreads_or(!empty)) {   // no value on the whole plane
+        for (int c = 0; c < NCH; ++c)
+            for (int e = threadIdx.x; e < D * H; e += NW * 32) out[(size_t)c * (D * D * H) + e] = make_float2(0.f, 0.f);
+        return;
+    }
     // y step 1, in place: items (c, j2, kz), kz fastest
     for (int t = threadIdx.x; t < NCH * N2 * H; t += NW * 32) {
         int kz, cj;
@@ -188,7 +203,6 @@ __device__ __forceinline__ void tpass_a(const PassA2 &a, int c0) {
     }
     __syncthreads();
     // y step 2: items (c, k1, kz), kz fastest -> S rows ky = k1 + N1 k2
-    float2 *out = a.S + (((size_t)b * a.nch + c0) * D + x) * (size_t)(D * H);
     for (int t = threadIdx.x; t < NCH * N1 * H; t += NW * 32) {
         const int kz = t % H, ck = t / H, k1 = ck % N1, c = ck / N1;
         const float2 *col = buf + c * CS + N2 * k1 * RS + kz;
