@@ -373,11 +373,12 @@ struct RegSide {
             k_rpass_b_line<NCH, N1, N2, PFA>
                 <<<dim3((D * H + kLineBThreads - 1) / kLineBThreads, nb), kLineBThreads, 0, st>>>(p);
         } else {
-            constexpr int nbx = (D * H + tb_cols<N1>() - 1) / tb_cols<N1>();
-            constexpr size_t sm = smem_tb<NCH, N1, N2>();
-            const int rper = tb_side<NCH>() * tb_rotations(nbx, nb / tb_side<NCH>());
+            constexpr BShape s = tb_shape<NCH, N1, N2, PFA>();
+            constexpr int nbx = (D * H + s.cols - 1) / s.cols;
+            constexpr size_t sm = smem_tb<NCH, N1, N2, PFA>();
+            const int rper = s.side * tb_rotations(nbx, nb / s.side);
             allow_smem(k_tpass_b<NCH, N1, N2, PFA>, sm);
-            k_tpass_b<NCH, N1, N2, PFA><<<dim3(nbx, (nb + rper - 1) / rper), tb_threads<N1>(), sm, st>>>(p, nb, rper);
+            k_tpass_b<NCH, N1, N2, PFA><<<dim3(nbx, (nb + rper - 1) / rper), s.threads, sm, st>>>(p, nb, rper);
         }
     }
     static void b_prob(int nb, cudaStream_t st, const PassB2 &p) {
@@ -385,12 +386,13 @@ struct RegSide {
             k_rpass_b_line_prob<N1, N2, PFA>
                 <<<dim3((D * H + kLineBThreads - 1) / kLineBThreads, nb, 2), kLineBThreads, 0, st>>>(p);
         } else {
-            constexpr int nbx = (D * H + tb_cols<N1>() - 1) / tb_cols<N1>();
-            constexpr size_t sm = smem_tb<4, N1, N2>();
-            const int rper = tb_rotations(2 * nbx, nb);
+            constexpr BShape s = tb_shape<4, N1, N2, PFA>();
+            constexpr int nbx = (D * H + s.cols - 1) / s.cols;
+            constexpr size_t sm = smem_tb<4, N1, N2, PFA>();
+            const int rper = s.side * tb_rotations(2 * nbx, nb / s.side);
             allow_smem(k_tpass_b_prob<N1, N2, PFA>, sm);
             k_tpass_b_prob<N1, N2, PFA>
-                <<<dim3(nbx, (nb + rper - 1) / rper, 2), tb_threads<N1>(), sm, st>>>(p, nb, rper);
+                <<<dim3(nbx, (nb + rper - 1) / rper, 2), s.threads, sm, st>>>(p, nb, rper);
         }
     }
     template <int NGRP, int SC>

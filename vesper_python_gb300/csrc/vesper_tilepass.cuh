@@ -230,36 +230,88 @@ __global__ void __launch_bounds__(ta_warps<N1, N2>() * 32, ta_ctas<kSrcProb, N1,
 }
 
 // ---- pass B -------------------------------------------------------------------
-template <int N1> __host__ __device__ constexpr int tb_cols() { return N1 >= 9 ? 16 : 32; }
-template <int N1> __host__ __device__ constexpr int tb_threads() { return (N1 * tb_cols<N1>() + 31) / 32 * 32; }
-// Rotations side by side in a CTA: one channel alone leaves most threads of steps 1 and 3 idle.
-template <int NCH> __host__ __device__ constexpr int tb_side() { return NCH == 1 ? 3 : 1; }
-template <int NCH, int N1, int N2>
+// Columns and threads per CTA, rotations side by side in it, CTAs that registers are
+// budgeted for.  The steps of N1 points have N2 items per column, channel and rotation,
+// those of N2 points N1, and every step ends at a barrier, so a shape leaves threads
+// idle (a step costs its rounds times its points); shared memory and registers (target
+// values, and a line of either step) decide how many CTAs cover one another's barriers.
+// The measured rates of 90 pairs of shapes go as busy^0.4 warps^0.36 CTAs^0.14, hence
+// the cubes; a shape other than a thread per item of the second forward step is taken
+// where that promises a tenth (a sixth for one channel, whose three rotations already
+// share the barriers: below that 42 and 100 lost), and never for PFA sides, which have
+// no fourth step (side 75: 1.61 either way).  Microseconds per rotation, a thread per
+// item before and after: mode V 48 0.69 -> 0.61, 54 1.18 -> 0.94, 72 4.19 -> 2.33,
+// 81 5.57 -> 3.16, 88 5.89 -> 3.88, 91 6.81 -> 4.37, 96 9.08 -> 6.30; one channel 39
+// 0.27 -> 0.18, 66 0.96 -> 0.65, 78 2.44 -> 1.13, 96 4.01 -> 2.01; prob mode 48 1.65 ->
+// 1.18, 72 8.8 -> 4.2, 78 12.2 -> 7.3, 96 19.0 -> 12.2.
+struct BShape {
+    int cols, side, threads, ctas;
+    double rank;
+};
+__host__ __device__ constexpr BShape tb_rank(int nch, int n1, int n2, int w, int nr, int t) {
+    const int its = (n1 * w + t - 1) / t, d = n1 * n2;
+    const int sm = nr * (nch + 1) * d * w * 8 + d * 8 + 1024;
+    const int held = 2 * its * nch * n2 + (n1 > 2 * n2 ? 2 * n1 : 4 * n2) + 32;
+    const int regs = held < 64 ? 64 : held > 255 ? 255 : (held + 7) / 8 * 8;
+    const int by_smem = 228 * 1024 / sm, by_regs = 65536 / (regs * t);
+    const int ctas = by_smem < by_regs ? by_smem : by_regs;
+    if (ctas < 1 || held > 200) return BShape{w, nr, t, 1, 0.0};
+    const double cost = (double)t * ((nr * nch * n2 * w + t - 1) / t * n1 + its * nr * nch * n2 +
+                                     (nr * n2 * w + t - 1) / t * n1 + its * nr * n2);
+    const double busy = nr * (double)(2 * nch + 2) * d * w / cost;
+    const double warps = ctas * t / 32 < 24 ? ctas * t / 32.0 : 24.0;
+    return BShape{w, nr, t, ctas, busy * busy * busy * warps * warps * warps * (ctas < 4 ? ctas : 4)};
+}
+template <int NCH, int N1, int N2, bool PFA>
+__host__ __device__ constexpr BShape tb_shape() {
+    constexpr int w0 = N1 >= 9 ? 16 : 32;
+    BShape best = tb_rank(NCH, N1, N2, w0, NCH == 1 ? 3 : 1, (N1 * w0 + 31) / 32 * 32);
+    best.ctas = 0;   // no budget
+    if (PFA) return best;
+    double least = (NCH == 1 ? 3.51 : 2.14) * best.rank;   // 1.17^8, 1.1^8
+    for (int w = 16; w <= 32; w += 16)
+        for (int nr = 1; nr <= 4; ++nr)
+            for (int t = 64; t <= 512; t += 32) {
+                const BShape s = tb_rank(NCH, N1, N2, w, nr, t);
+                if (s.rank > least) {
+                    best = s;
+                    least = 1.0001 * s.rank;
+                }
+            }
+    return best;
+}
+// SH: the channels that the shape is chosen for (prob mode's two kinds share a launch)
+template <int SH, int N1, int N2, bool PFA>
 __host__ __device__ constexpr size_t smem_tb() {
+    constexpr BShape s = tb_shape<SH, N1, N2, PFA>();
     return (size_t)((N1 * N2 + 1) / 2 * 2) * sizeof(float2) +
-           (size_t)tb_side<NCH>() * (NCH + 1) * N1 * N2 * tb_cols<N1>() * sizeof(float2);
+           (size_t)s.side * (SH + 1) * N1 * N2 * s.cols * sizeof(float2);
 }
 
-template <int NCH, int N1, int N2, bool PFA>
+template <int NCH, int SH, int N1, int N2, bool PFA>
 __device__ __forceinline__ void tpass_b(const PassB2 &a, int c0, int grp, int nb, int rper) {
-    constexpr int D = N1 * N2, H = D / 2 + 1, dH = D * H, W = tb_cols<N1>(), TB = tb_threads<N1>();
-    constexpr int NR = tb_side<NCH>();
+    constexpr BShape shape = tb_shape<SH, N1, N2, PFA>();
+    constexpr int D = N1 * N2, H = D / 2 + 1, dH = D * H, W = shape.cols, TB = shape.threads, NR = shape.side;
+    constexpr int IT = (N1 * W + TB - 1) / TB;   // items of step 2 per thread
     extern __shared__ __align__(16) unsigned char smem[];
     float2 *twn = (float2 *)smem;
     float2 *buf = twn + (D + 1) / 2 * 2;              // [NR][NCH][D][W]
     float2 *pbuf = buf + (size_t)NR * NCH * D * W;    // [NR][D][W]
     const int j0 = blockIdx.x * W, b0 = blockIdx.y * rper, b1 = min(nb, b0 + rper);
     twiddles_n(D, twn);
-    // the thread's target values: item (k1, w) of step 2, for every rotation
-    const int w2 = threadIdx.x % W, k1_ = threadIdx.x / W;
-    const bool on2 = threadIdx.x < N1 * W && j0 + w2 < dH;
-    float2 tv[NCH][N2];
+    // the thread's target values: items (k1, w) of step 2, for every rotation
+    float2 tv[IT][NCH][N2];
 #pragma unroll
-    for (int c = 0; c < NCH; ++c)
+    for (int i = 0; i < IT; ++i) {
+        const int t = threadIdx.x + i * TB, w = t % W, k1 = t / W;
+        const bool on = t < N1 * W && j0 + w < dH;
 #pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2)
-            tv[c][k2] = on2 ? __ldg(a.T + (size_t)(c0 + c) * D * dH + (size_t)(k1_ + N1 * k2) * dH + j0 + w2)
-                            : make_float2(0.f, 0.f);
+        for (int c = 0; c < NCH; ++c)
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2)
+                tv[i][c][k2] = on ? __ldg(a.T + (size_t)(c0 + c) * D * dH + (size_t)(k1 + N1 * k2) * dH + j0 + w)
+                                  : make_float2(0.f, 0.f);
+    }
     __syncthreads();
     for (int b = b0; b < b1; b += NR) {
         const float2 *src = a.S + ((size_t)b * a.nch + c0) * D * dH + j0;
@@ -279,27 +331,31 @@ __device__ __forceinline__ void tpass_b(const PassB2 &a, int c0, int grp, int nb
         __syncthreads();
         // forward step 2, product with conj(T), channel sum; PFA: inverse step 2 with
         // conjugate twiddles into pbuf rows k1 + N1 j2, else the sums themselves there
-        if (threadIdx.x < N1 * W) {
 #pragma unroll
-            for (int rr = 0; rr < NR; ++rr) {
-                float2 acc[N2];
+        for (int i = 0; i < IT; ++i) {
+            const int t = threadIdx.x + i * TB, w = t % W, k1 = t / W;
+            if (t < N1 * W) {
 #pragma unroll
-                for (int k2 = 0; k2 < N2; ++k2) acc[k2] = make_float2(0.f, 0.f);
+                for (int rr = 0; rr < NR; ++rr) {
+                    float2 acc[N2];
 #pragma unroll
-                for (int c = 0; c < NCH; ++c) {
-                    const float2 *col = buf + (size_t)((rr * NCH + c) * D + N2 * k1_) * W + w2;
-                    float2 u[N2];
+                    for (int k2 = 0; k2 < N2; ++k2) acc[k2] = make_float2(0.f, 0.f);
 #pragma unroll
-                    for (int j2 = 0; j2 < N2; ++j2) u[j2] = col[j2 * W];
-                    line_dft<N2, D, false, PFA>(u, twn);
+                    for (int c = 0; c < NCH; ++c) {
+                        const float2 *col = buf + (size_t)((rr * NCH + c) * D + N2 * k1) * W + w;
+                        float2 u[N2];
 #pragma unroll
-                    for (int k2 = 0; k2 < N2; ++k2) acc[k2] = cadd(acc[k2], cmul(tv[c][k2], u[k2]));
+                        for (int j2 = 0; j2 < N2; ++j2) u[j2] = col[j2 * W];
+                        line_dft<N2, D, false, PFA>(u, twn);
+#pragma unroll
+                        for (int k2 = 0; k2 < N2; ++k2) acc[k2] = cadd(acc[k2], cmul(tv[i][c][k2], u[k2]));
+                    }
+                    if constexpr (PFA) rdft<N2, true>(acc);
+                    float2 *col = pbuf + (rr * D + k1) * W + w;
+#pragma unroll
+                    for (int j2 = 0; j2 < N2; ++j2)
+                        col[N1 * j2 * W] = (PFA && k1 && j2) ? cmulc(acc[j2], twn[j2 * k1]) : acc[j2];
                 }
-                if constexpr (PFA) rdft<N2, true>(acc);
-                float2 *col = pbuf + (rr * D + k1_) * W + w2;
-#pragma unroll
-                for (int j2 = 0; j2 < N2; ++j2)
-                    col[N1 * j2 * W] = (PFA && k1_ && j2) ? cmulc(acc[j2], twn[j2 * k1_]) : acc[j2];
             }
         }
         __syncthreads();
@@ -318,18 +374,22 @@ __device__ __forceinline__ void tpass_b(const PassB2 &a, int c0, int grp, int nb
                 for (int k1 = 0; k1 < N1; ++k1) col[N2 * k1 * W] = (k1 && j2) ? twiddle<true>(v[k1], twn[j2 * k1]) : v[k1];
             }
             __syncthreads();
-            if (threadIdx.x < N1 * W) {
 #pragma unroll
-                for (int rr = 0; rr < NR; ++rr) {
-                    const float2 *col = pbuf + (rr * D + N2 * k1_) * W + w2;
-                    float2 u[N2];
+            for (int i = 0; i < IT; ++i) {
+                const int t = threadIdx.x + i * TB, w = t % W, k1 = t / W;
+                if (t < N1 * W) {
 #pragma unroll
-                    for (int j2 = 0; j2 < N2; ++j2) u[j2] = col[j2 * W];
-                    rdft_plan<N2, true, N1>(u, twn);
-                    if (on2 && (NR == 1 || b + rr < b1))
+                    for (int rr = 0; rr < NR; ++rr) {
+                        const float2 *col = pbuf + (rr * D + N2 * k1) * W + w;
+                        float2 u[N2];
 #pragma unroll
-                        for (int k2 = 0; k2 < N2; ++k2)
-                            dst[((size_t)rr * a.ngrp * D + k1_ + N1 * k2) * dH + w2] = u[k2];
+                        for (int j2 = 0; j2 < N2; ++j2) u[j2] = col[j2 * W];
+                        rdft_plan<N2, true, N1>(u, twn);
+                        if (j0 + w < dH && (NR == 1 || b + rr < b1))
+#pragma unroll
+                            for (int k2 = 0; k2 < N2; ++k2)
+                                dst[((size_t)rr * a.ngrp * D + k1 + N1 * k2) * dH + w] = u[k2];
+                    }
                 }
             }
             continue;
@@ -351,15 +411,17 @@ __device__ __forceinline__ void tpass_b(const PassB2 &a, int c0, int grp, int nb
 }
 
 template <int NCH, int N1, int N2, bool PFA>
-__global__ void __launch_bounds__(tb_threads<N1>()) k_tpass_b(const PassB2 a, int nb, int rper) {
-    tpass_b<NCH, N1, N2, PFA>(a, 0, 0, nb, rper);
+__global__ void __launch_bounds__(tb_shape<NCH, N1, N2, PFA>().threads, tb_shape<NCH, N1, N2, PFA>().ctas)
+    k_tpass_b(const PassB2 a, int nb, int rper) {
+    tpass_b<NCH, NCH, N1, N2, PFA>(a, 0, 0, nb, rper);
 }
 template <int N1, int N2, bool PFA>
-__global__ void __launch_bounds__(tb_threads<N1>()) k_tpass_b_prob(const PassB2 a, int nb, int rper) {
+__global__ void __launch_bounds__(tb_shape<4, N1, N2, PFA>().threads, tb_shape<4, N1, N2, PFA>().ctas)
+    k_tpass_b_prob(const PassB2 a, int nb, int rper) {
     if (blockIdx.z == 0)
-        tpass_b<3, N1, N2, PFA>(a, 0, 0, nb, rper);
+        tpass_b<3, 4, N1, N2, PFA>(a, 0, 0, nb, rper);
     else
-        tpass_b<4, N1, N2, PFA>(a, 3, 1, nb, rper);
+        tpass_b<4, 4, N1, N2, PFA>(a, 3, 1, nb, rper);
 }
 
 // ---- pass C -------------------------------------------------------------------
@@ -449,7 +511,7 @@ __global__ void __launch_bounds__(tc_warps<N1, N2>() * 32) k_tpass_c(const PassC
     // greatest scores, as offsets from the item's first voxel (half the instructions of
     // a 64-bit key per voxel); merged as keys once per item.
     // float_order as a signed value: the sum makes -0 a +0.
-    int top[SC], at[SC];
+    int top[SC] = {}, at[SC] = {};
     auto take = [&](int s, float v, int off) {
         const int i = __float_as_int(__fadd_rn(v, 0.f)), o = i ^ (i >> 31 & 0x7fffffff);
         if (o > top[s]) {
