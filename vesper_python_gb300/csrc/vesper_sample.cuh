@@ -42,8 +42,8 @@ __device__ __forceinline__ void store_reach(float r2, unsigned *reach) {   // wh
     if (m && (threadIdx.x & 31) == 0) atomicMax(reach, m);
 }
 
-// reach (or null): of the vectors or values, and of the probabilities
-template <int MODE>
+// REACH: also finds that of the vectors or values, and of the probabilities
+template <int MODE, bool REACH>
 __global__ void k_pack(const double *data, const float *vec, const float *probs, int d, double ave, float4 *q4,
                        float4 *p4, unsigned *reach) {
     const size_t n = (size_t)d * d * d;
@@ -59,30 +59,30 @@ __global__ void k_pack(const double *data, const float *vec, const float *probs,
             o = make_float4(query_value<MODE>(v, ave), 0.f, 0.f, m);
         }
         q4[i] = o;
-        if (reach) voxel_reach(i, d, m != 0.f, r2);
+        if constexpr (REACH) voxel_reach(i, d, m != 0.f, r2);
         if (MODE == VESPER_MODE_PROB) {
             const float4 p = make_float4(probs[i], probs[n + i], probs[2 * n + i], probs[3 * n + i]);
             p4[i] = p;
-            if (reach) voxel_reach(i, d, p.x != 0.f || p.y != 0.f || p.z != 0.f || p.w != 0.f, rp);
+            if constexpr (REACH) voxel_reach(i, d, p.x != 0.f || p.y != 0.f || p.z != 0.f || p.w != 0.f, rp);
         }
     }
-    if (reach) store_reach(r2, reach);
-    if (MODE == VESPER_MODE_PROB && reach) store_reach(rp, reach + 1);
+    if constexpr (REACH) store_reach(r2, reach);
+    if constexpr (REACH && MODE == VESPER_MODE_PROB) store_reach(rp, reach + 1);
 }
 
 // The value of the scalar modes alone (4 bytes a voxel: a gather's cache lines
 // hold four times as many), for the register passes; it is zero wherever the
 // density is.
-template <int MODE>
+template <int MODE, bool REACH>
 __global__ void k_pack_value(const double *data, int d, double ave, float *q1, unsigned *reach) {
     const size_t n = (size_t)d * d * d;
     float r2 = 0.f;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double v = data[i];
         q1[i] = query_value<MODE>(v, ave);
-        if (reach) voxel_reach(i, d, v != 0.0, r2);
+        if constexpr (REACH) voxel_reach(i, d, v != 0.0, r2);
     }
-    if (reach) store_reach(r2, reach);
+    if constexpr (REACH) store_reach(r2, reach);
 }
 
 // ---- gather -----------------------------------------------------------------
