@@ -291,7 +291,7 @@ def kernel_names(dev, dim, mode):
     path = vg.search_plan(dim, mode, 0, 1, None, dev)[0]
     if path == 2:
         return {"search": "k_fused"}
-    pre = "k_rpass_" if path == 1 else "k_pass_"
+    pre = "k_pass_" if path != 1 else "k_tpass_" if dim > 32 else "k_rpass_"
     return {"pass_a": pre + "a", "pass_b": pre + "b", "pass_c": pre + "c"}
 
 
@@ -747,8 +747,8 @@ def run_uneven(args, sub=False):
     pct = lambda a, q: round(float(np.percentile(a, q)), 3)
     # pass roofline over the whole batch (every side's register / radix-pass
     # searches; the fused sides' time counts in whole_search only)
-    roof = search_roofline(prof, dev, clocks, {"pass_a": "k_rpass_a / k_pass_a", "pass_b": "k_rpass_b / k_pass_b",
-                                               "pass_c": "k_rpass_c / k_pass_c", "search": "k_fused"})
+    roof = search_roofline(prof, dev, clocks, {"pass_a": "k_rpass_a_line / k_tpass_a / k_pass_a", "pass_b": "k_rpass_b_line / k_tpass_b / k_pass_b",
+                                               "pass_c": "k_rpass_c_line / k_tpass_c / k_pass_c", "search": "k_fused"})
     line = {
         "metric": METRIC, "value": round(n / (ms / 1e3), 4), "unit": UNIT, "n_gpus": world, "steps": steps,
         "warmup": warmup, "ms_per_step": round(ms, 3), "higher_is_better": True, "scaling": "weak",

@@ -8,9 +8,9 @@ rotations for every candidate of
   cchunk     channels gathered and transformed per pass-A block
   W          spectrum columns per pass-B block
 
-and keeps the fastest.  The kernel family (register two-step FFT where it is
-compiled for the side, radix-stage otherwise) is fixed by the side, so every
-candidate computes bit-identical results and the choice only changes speed.
+and keeps the fastest (the register passes take only the batch; their other
+shapes are fixed per side).  The kernel family (register passes at sides 25 to
+100, radix-stage otherwise) is fixed by the side, so every candidate computes bit-identical results and the choice only changes speed.
 Results are cached per process and, unless VESPER_AUTOTUNE_CACHE is set to
 an empty string, in a JSON file (default ~/.cache/vesper_gb300/autotune.json).
 """
