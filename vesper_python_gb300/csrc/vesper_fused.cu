@@ -22,8 +22,6 @@
 
 namespace vg {
 
-constexpr int kFusedThreads = 256;
-
 template <int D>
 struct FGeom {
     static constexpr int H = D / 2 + 1;
@@ -47,17 +45,31 @@ struct FusedArgs {
     unsigned long long *keys;
 };
 
-// CTAs per SM the register budget is sized for, as many as the side's shared
-// volume allows without spilling: 4 (64 registers) up to side 13, 3 up to
-// 15, 2 for 16 to 20, 1 above and for the Laplacian mode (its float64
-// stencil needs the registers).
-template <int MODE, int D>
-constexpr int fused_ctas() {
-    return MODE == VESPER_MODE_LAPLACIAN ? 1 : D <= 13 ? 4 : D <= 15 ? 3 : D <= 20 ? 2 : 1;
+// Threads per CTA and the CTAs per SM that registers are budgeted for.  Where shared
+// memory leaves two CTAs or one (mode V from side 18 and from side 21), more threads are
+// the only way to more warps: 320 (96 registers) and 512 (128), nothing spills.  Measured,
+// 1,008 rotations, us per rotation, 256 threads before: side 21 0.361 -> 0.241, 22 0.215
+// -> 0.163, 24 0.243 -> 0.185, 18 0.095 -> 0.089, 20 0.111 -> 0.108 (124 rotations: 0.323
+// -> 0.273).  Below, 256 threads and as many CTAs as registers allow without spilling (4
+// up to side 13, 3 up to 15, 2 at 16): fewer threads and more CTAs, whose steps leave
+// fewer lanes idle, gained up to 10 % for a thousand rotations (side 10) but lost at
+// others (14 0.048 -> 0.056) and lost half for a few (side 13, 124 rotations).  The
+// Laplacian mode's float64 stencil needs the registers: one CTA's budget.
+struct FShape {
+    int threads, ctas;
+};
+template <int MODE, int NCH, int D>
+constexpr FShape fused_shape() {
+    constexpr int by_smem = (int)(228 * 1024 / (fused_smem<NCH, D>() + 1024));
+    if (MODE == VESPER_MODE_LAPLACIAN) return FShape{256, 1};
+    if (by_smem == 1) return FShape{512, 1};
+    if (by_smem == 2) return FShape{320, 2};
+    return FShape{256, D <= 13 ? 4 : D <= 15 ? 3 : 2};
 }
 
 template <int MODE, int NCH, int D>
-__global__ void __launch_bounds__(kFusedThreads, fused_ctas<MODE, D>()) k_fused(const FusedArgs a) {
+__global__ void __launch_bounds__(fused_shape<MODE, NCH, D>().threads, fused_shape<MODE, NCH, D>().ctas)
+    k_fused(const FusedArgs a) {
     using G = FGeom<D>;
     constexpr int H = G::H, NP = G::NP, Hp = G::Hp, RS = G::RS, CS = G::CS;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -203,6 +215,7 @@ __global__ void __launch_bounds__(kFusedThreads, fused_ctas<MODE, D>()) k_fused(
 template <int MODE, int NCH, int D>
 static int launch_fused(const FusedArgs &a, cudaStream_t st) {
     constexpr size_t sm = fused_smem<NCH, D>();
+    constexpr int threads = fused_shape<MODE, NCH, D>().threads;
     if (sm > (size_t)smem_limit()) return fail(VESPER_ERR_UNSUPPORTED, "fused search: side %d too large", D);
     allow_smem(k_fused<MODE, NCH, D>, sm);
     // resident CTAs of the whole GPU, queried once per device
@@ -218,14 +231,14 @@ static int launch_fused(const FusedArgs &a, cudaStream_t st) {
     }
     if (cap == 0) {
         int per_sm = 0, nsm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused<MODE, NCH, D>, kFusedThreads, sm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused<MODE, NCH, D>, threads, sm);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         cap = std::max(per_sm, 1) * std::max(nsm, 1);
         std::lock_guard<std::mutex> g(mu);
         slots[dev] = cap;
     }
     const int grid = std::max(1, std::min(a.nrot, cap));
-    k_fused<MODE, NCH, D><<<grid, kFusedThreads, sm, st>>>(a);
+    k_fused<MODE, NCH, D><<<grid, threads, sm, st>>>(a);
     VG_CHECK_LAUNCH("k_fused");
     return VESPER_OK;
 }
