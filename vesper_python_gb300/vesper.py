@@ -64,6 +64,8 @@ class Device:
         self.index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         self.lib = _native.load()
         self._ws = {}
+        self._captured = set()   # keys whose buffer a stream capture has used
+        self._kept = []          # such buffers that a larger one has replaced
 
     @property
     def stream(self):
@@ -73,12 +75,23 @@ class Device:
 
     def workspace(self, key, nbytes):
         """Scratch buffer for ``key`` on the current stream (work on different
-        streams never shares scratch)."""
+        streams never shares scratch).  A captured graph holds the buffer's
+        address and no reference, so a buffer that a capture has used lives as
+        long as the Device, also once a call that needs more has replaced it;
+        the replacement is at least twice as large, so that the replaced ones
+        of a key never hold more than the one in use."""
         key = key + (_raw_stream(self.index),)
         buf = self._ws.get(key)
         if buf is None or buf.numel() < nbytes:
-            buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=self.device)
+            nbytes = max(int(nbytes), 256)
+            if key in self._captured:
+                self._kept.append(buf)
+                self._captured.discard(key)
+                nbytes = max(nbytes, 2 * buf.numel())
+            buf = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
             self._ws[key] = buf
+        if torch.cuda.is_current_stream_capturing():
+            self._captured.add(key)
         return buf
 
     def to_dev_async(self, a):
