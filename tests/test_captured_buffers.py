@@ -78,6 +78,6 @@ def test_replay_after_a_larger_eager_call(dev):
         assert al.graph_captures == 2
         for a, b in zip(ref, again):
             assert (a.dim, a.std, a.ave, a.top) == (b.dim, b.std, b.ave, b.top)
-            assert [(m.angle, m.vec_score, m.vec_trans, m.dot_score, m.cc) for m in a.models] == \\
+            assert [(m.angle, m.vec_score, m.vec_trans, m.dot_score, m.cc) for m in a.models] == \
                 [(m.angle, m.vec_score, m.vec_trans, m.dot_score, m.cc) for m in b.models]
         assert all(bool((f == 77).all()) for f in fill)
