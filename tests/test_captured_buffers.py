@@ -1,8 +1,13 @@
 """What a captured graph reads and writes stays allocated as long as the graph can be replayed: the
-scratch of Device.workspace (without a GPU the allocations are host tensors and the capture is a flag)."""
+weights of the proposal network, the scratch of Device.workspace (without a GPU the allocations are host tensors and the capture is a flag)."""
+import contextlib
+import types
+
+import numpy as np
 import pytest
 import torch
 
+from vesper_python_gb300 import align
 from vesper_python_gb300 import vesper as vg
 
 
@@ -57,11 +62,46 @@ def test_scratch_without_a_capture_is_given_back_and_kept_scratch_is_bounded(mon
         assert sum(t.numel() for t in dev._kept) <= buf.numel() < 2 * nbytes + 8000
 
 
+def test_captured_stage_keeps_the_networks_weights(monkeypatch):
+    """Other weights, of the same network or of one that takes its place, are another signature, and the weights
+    that a captured stage reads are not given back."""
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", lambda: types.SimpleNamespace(replay=lambda: None))
+    monkeypatch.setattr(torch.cuda, "graph", lambda g: contextlib.nullcontext())
+    al = align.Aligner(types.SimpleNamespace(lib=None))
+    monkeypatch.setattr(al, "_global_stage", lambda P, p, mats, nang: (None, None))
+    m = torch.zeros(4, 4, 4)
+    st = align._Pair(m, m, 1.0, 1.0, np.zeros(3), np.zeros(3))
+    st.dim, st.no1, st.no2, st.o1, st.o2 = 8, np.zeros(3), np.zeros(3), np.zeros(3), np.zeros(3)
+    for k in al._STAGE_FIELDS:
+        if k != "launches":
+            setattr(st, k, None)
+
+    def weights():
+        return [torch.zeros(300), torch.zeros(500)]
+
+    net = types.SimpleNamespace(Wbf=weights(), b=weights())
+    p = align.AlignParams(proposal=net)
+    used = set()
+    for captures in (1, 2, 3):
+        at = {t.data_ptr() for t in net.Wbf + net.b}
+        assert not (at & used)           # the ones before are still held
+        used |= at
+        for _ in range(2):
+            al._global_stage_graph([st], p, m, 8)
+            assert al.graph_captures == captures
+        if captures == 1:
+            del net.Wbf, net.b           # load_state_dict
+            net.Wbf, net.b = weights(), weights()
+        else:
+            p.proposal = net = None      # another network
+            p.proposal = net = types.SimpleNamespace(Wbf=weights(), b=weights())
+
+
 @pytest.mark.gpu
 def test_replay_after_a_larger_eager_call(dev):
     """A graph with 270 refinement slots per pair, then eager calls with 1,080 on the same side streams, then
     tensors over whatever was given back: the replay gives its results again and the tensors keep their values."""
-    from vesper_python_gb300 import align, synth
+    from vesper_python_gb300 import synth
     items = []
     for i in range(3):
         pair = synth.make_pair(60 + i, 64, 40, 18.0)

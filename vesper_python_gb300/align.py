@@ -657,7 +657,8 @@ class Aligner:
         (input addresses and shapes, grid geometry, parameters): a repeated
         batch replays one graph instead of its hundreds of launches.  A new
         signature runs the stage once eagerly (autotuning, first launches),
-        then captures it."""
+        then captures it.  The entry keeps the network's weights: the graph reads
+        them at their addresses, which name them in the signature."""
         sig = self._batch_sig(P, p, mats)
         ent = self._graphs.get(sig)
         if ent is None:
@@ -676,9 +677,9 @@ class Aligner:
                 sv["launches"] = st.launches - b0          # launches inside the graph
                 st.launches = b0
                 saved.append(sv)
-            ent = self._graphs[sig] = (g, stats, saved)
+            ent = self._graphs[sig] = (g, stats, saved, self._weights(p))
             self.graph_captures += 1
-        g, stats, saved = ent
+        g, stats, saved, _ = ent
         self._mark("global")
         g.replay()
         for st, sv in zip(P, saved):
@@ -691,14 +692,20 @@ class Aligner:
         return stats
 
     @staticmethod
+    def _weights(p):
+        """The tensors of the proposal network that a captured stage reads."""
+        return [] if p.proposal is None else [*p.proposal.Wbf, *p.proposal.b]
+
+    @staticmethod
     def _batch_sig(P, p, mats):
         """What a captured stage depends on: input addresses and shapes, grid
-        geometry, parameters, the angle grid."""
+        geometry, parameters, the network's weights, the angle grid."""
         return (tuple((st.src1.data_ptr(), st.src2.data_ptr(), tuple(st.src1.shape), tuple(st.src2.shape), st.dim,
                        *np.asarray(st.no1, np.float64).tolist(), *np.asarray(st.no2, np.float64).tolist(),
                        float(st.width1), float(st.width2), *np.asarray(st.o1).tolist(), *np.asarray(st.o2).tolist())
                       for st in P),
-                (p.t, p.T, p.g, p.s, p.A, p.N, p.mode, p.batch, id(p.proposal), p.proposal_frac, p.proposal_pool),
+                (p.t, p.T, p.g, p.s, p.A, p.N, p.mode, p.batch, tuple(t.data_ptr() for t in Aligner._weights(p)),
+                 p.proposal_frac, p.proposal_pool),
                 mats.data_ptr())
 
     # ---- refinement and rescoring on the device ---------------------------------
