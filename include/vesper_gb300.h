@@ -302,7 +302,7 @@ int vesper_rescore_batch_dev(const double *tdata, const float *tvec, const doubl
  *
  * vesper_refine_pick: one pair's slots after their search (scores float and
  * lin int32 [nslot][nscore], column 0 used): the stable top-N over the valid
- * slots (the others read -inf; ties to the lower slot; -1 past the slots) in
+ * slots (ties to the lower slot; -1 where no valid slot is left) in
  * rtop int32 [topn], and per pick (slot 0 standing in for -1) its row int64,
  * score float, lin int64, rotation mats float [topn][3][3] = lattice[row] and
  * trans int32 [topn][3] = (lin / d^2, lin / d % d, lin % d), each t > d/2

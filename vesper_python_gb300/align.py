@@ -713,8 +713,7 @@ class Aligner:
     # 5-degree lattice in the reference's meshgrid order, kept where x < 360,
     # y < 360 and z < 180 and wrapped by +360 where negative (:689-713).  Every
     # pair gets N x 27 slots in that order, the slots the filter drops marked
-    # invalid and left out of the top-N (their score reads -inf), so the stable
-    # top-N over the slots is the reference's over its list, duplicates
+    # invalid and left out of the top-N, so the stable top-N over the slots is the reference's over its list, duplicates
     # included.  The models' rotations are rows of the lattice table, their
     # translations come from the search's linear index, and the float64
     # rescoring reads the target statistics from the device: nothing in the

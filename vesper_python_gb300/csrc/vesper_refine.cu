@@ -36,7 +36,7 @@ __global__ void k_refine_slots(const int64_t *tg, int n, int N, const int64_t *g
 }
 
 // One pair: the stable top-N of scores[s nscore] over the slots s with
-// valid[s] (the others read -inf), ties to the lower slot, -1 past the slots;
+// valid[s], ties to the lower slot, -1 where no such slot is left;
 // then per pick k (slot 0 standing in for -1): the slot's lattice row, its
 // score, its linear translation lin, the row's rotation matrix, and
 // (lin / d^2, lin / d % d, lin % d) with each t > d / 2 taken as t - d.
@@ -57,9 +57,8 @@ __global__ void __launch_bounds__(kPickThreads) k_refine_pick(const float *score
     for (int k = 0; k < topn; ++k) {
         unsigned long long best = 0ull;
         for (int i = threadIdx.x; i < nslot; i += blockDim.x) {
-            if (taken[i >> 5] & (1u << (i & 31))) continue;
-            const float s = valid[i] ? scores[(size_t)i * nscore] : -INFINITY;
-            best = max(best, make_key(s, (uint32_t)i));
+            if (!valid[i] || (taken[i >> 5] & (1u << (i & 31)))) continue;
+            best = max(best, make_key(scores[(size_t)i * nscore], (uint32_t)i));
         }
         best = warp_max_u64(best);
         if (lane == 0) red[warp] = best;
