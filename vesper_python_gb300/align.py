@@ -257,6 +257,8 @@ class Aligner:
         if n == 0:
             return []
         P = [_Pair(*it) for it in items]
+        for i, st in enumerate(P):
+            st.index = i
         # ---- 1. threshold + radius (device), grid sizing (host) ----------------
         self._mark("prepare")
         prep = torch.empty((n, 4), dtype=torch.int64, device=dev.device)
@@ -308,11 +310,11 @@ class Aligner:
         device_late = (graph or late_eager) and mode not in ("PCC", "CC") and p.A > 5.0 and self.group is None and \
             self._grid_rows(p.A, angle_comb) is not None
 
-        def late_stage():
-            if graph:
+        def late_stage(sts=P):
+            if graph:       # the graph holds every pair
                 self._late_stage_graph(P, p, stats, mats)
             else:
-                self._late_stage(P, p, stats)
+                self._late_stage(sts, p, stats if sts is P else stats[[st.index for st in sts]])
 
         def global_results():
             # the global results go to the host while the refinement runs
@@ -324,10 +326,10 @@ class Aligner:
         if p.proposal is not None:
             zdev = torch.stack([st.z for st in P])
             if device_late:
-                # the refinement graph is launched before the flatness test is
-                # read back, so the device does not wait for the host; a pair
-                # that falls back to the exhaustive search (rare) is refined
-                # again below
+                # the refinement is launched before the flatness test is read
+                # back, so the device does not wait for the host; a pair that
+                # falls back to the exhaustive search (rare) is refined again
+                # below (in the graph form with the others)
                 zh = self._fetch_start([[zdev]], slot=2)
                 gh = global_results()
                 late_stage()
@@ -343,7 +345,7 @@ class Aligner:
                 st.tg.copy_(st.top.to(st.tg.dtype))     # top grid indices, read by the device late stage
             if redo and device_late:
                 gh = global_results()
-                late_stage()
+                late_stage(redo)
             self.proposal_info = {"subset": int(np.ceil(p.proposal_frac * nang)), "z": [float(z) for z in zs],
                                   "fallback": [bool(st.fallback) for st in P]}
         else:
@@ -793,9 +795,8 @@ class Aligner:
                     c_(gv.data_ptr()), d, c_(trd.data_ptr()), N, c_(st.res.data_ptr()), c_(ws.data_ptr()),
                     ws.numel(), dev.stream))
                 if self.pair_events is not None and not capturing:
-                    e = torch.cuda.Event(enable_timing=True)
-                    e.record()
-                    self.pair_events.append(e)
+                    st.done = torch.cuda.Event(enable_timing=True)
+                    st.done.record()
             st.launches += self._search_launches(d, mode, N * 27, p.batch) + 7
             if not capturing:
                 for tt in (st.rtop, st.r_rows, st.r_score, st.r_lin, st.res):
@@ -842,7 +843,8 @@ class Aligner:
         if self.pair_events is not None:   # every pair ends with the graph
             e = torch.cuda.Event(enable_timing=True)
             e.record()
-            self.pair_events.extend([e] * len(P))
+            for st in P:
+                st.done = e
         self.graph_replays += 1
 
     def _finish_device_late(self, P, p, gh, angle_comb):
@@ -853,6 +855,8 @@ class Aligner:
         PCC never come here, so every score scale is 1."""
         mode = p.mode
         assert mode not in ("CC", "PCC")
+        if self.pair_events is not None:
+            self.pair_events.extend(st.done for st in P)
         self._mark("results")
         late = self._fetch_start([[st.rtop, st.r_rows, st.r_score, st.r_lin, st.res] for st in P], slot=1)
         glob = self._fetch_finish(gh)
