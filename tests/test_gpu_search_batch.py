@@ -1,0 +1,39 @@
+"""The batch that batch = 0 takes, by the launches that vesper_search_profile counts: the library's default
+where the workspace holds it, else the largest that the workspace holds."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode,d", [("VecProduct", 48), ("prob", 48), ("Laplacian", 36), ("CC", 36), ("CC", 21),
+                                    ("VecProduct", 16)])
+@pytest.mark.parametrize("room", ["full", "least"])
+def test_profile_counts_the_launches_made(dev, mode, d, room):
+    from vesper_python_gb300 import _native
+    from vesper_python_gb300 import vesper as vg
+    n, code, prob = 500, vg.MODE_CODES[mode], mode == "prob"
+    per = (9 if prob else 4 if mode == "VecProduct" else 2) * d * d * (d // 2 + 1) * 8
+    base = min((64 << 20) // per, 2048)
+    nbytes = _native.size_query("vesper_search_workspace_size", d, code, 0 if room == "full" else base, n)
+    data, vec = torch.rand((d, d, d), dtype=torch.float64, device=dev.device), torch.rand((d, d, d, 3), device=dev.device)
+    probs = torch.rand((4, d, d, d), device=dev.device) if prob else None
+    spec = vg.target_spectra_device(data, vec, mode, 0.0, probs=probs, dev=dev)
+    mats = dev.to_dev(vg.rot_matrices(vg.calc_angle_comb(30.0)[:n]))
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev.device)
+    sc = torch.empty((n, 2 if prob else 1), device=dev.device)
+    ln = torch.empty((n, 2 if prob else 1), dtype=torch.int32, device=dev.device)
+    ms, nl = (ctypes.c_float * 4)(), (ctypes.c_int * 4)()
+    p = lambda t: ctypes.c_void_p(t.data_ptr() if t is not None else None)  # noqa: E731
+    _native.check(dev.lib.vesper_search_profile(p(spec), p(data), p(vec), p(probs), d, code, 0.0, p(mats), n, None, p(sc),
+                                                p(ln), 0, p(ws), nbytes, dev.stream, ms, nl, None))
+    if vg.search_plan(d, mode, 0, 1, None, dev)[0] == 2:
+        want = [1, 0, 0, 1]                                     # the fused kernel
+    else:
+        total = per + (d ** 3 * 8 if mode == "Laplacian" else 0)
+        full = max(base, min(n, 256, (1 << 30) // total))
+        steps = -(-n // (full if room == "full" else base))
+        want = [steps, steps, steps, 1]
+    assert list(nl) == want

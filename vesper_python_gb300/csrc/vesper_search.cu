@@ -107,6 +107,7 @@ struct PassTimer {
     cudaEvent_t ev[kRing][4][2];
     bool used[kRing][4];
     float ms[4];
+    int n[4];   // launches of each pass
 };
 
 template <int MODE, int NCH>
@@ -349,7 +350,10 @@ static int search_impl(const void *spectra, const double *data, const float *vec
         if (!tm) return;
         if (edge == 0 && tm->used[slot][pass]) drain(slot);
         cudaEventRecord(tm->ev[slot][pass][edge], st);
-        if (edge == 1) tm->used[slot][pass] = true;
+        if (edge == 1) {
+            tm->used[slot][pass] = true;
+            ++tm->n[pass];
+        }
     };
     if (fused) {
         int frc = VESPER_OK;
@@ -467,17 +471,16 @@ extern "C" int vesper_search_profile(const void *spectra, const double *data, co
     }
     for (int sl = 0; sl < kRing; ++sl)
         for (int p = 0; p < 4; ++p) tm.used[sl][p] = false;
-    for (int p = 0; p < 4; ++p) tm.ms[p] = 0.f;
+    for (int p = 0; p < 4; ++p) {
+        tm.ms[p] = 0.f;
+        tm.n[p] = 0;
+    }
     const int rc = search_impl(spectra, data, vec, probs, dim, mode, ave, rotmats, nrot, mix, scores_out, lin_out,
                                batch, workspace, workspace_bytes, stream, &tm, opts);
-    for (int p = 0; p < 4; ++p) pass_ms[p] = tm.ms[p];
-    int path = 0, launches = 0;
-    vesper_search_plan(dim, mode, batch, nrot, opts, &path, &launches);
-    if (batch <= 0) batch = default_batch(dim, mode, nrot);
-    const int nb = nrot > 0 ? (nrot + batch - 1) / batch : 0;
-    pass_launches[0] = path == 2 ? (nrot > 0) : nb;
-    pass_launches[1] = pass_launches[2] = path == 2 ? 0 : nb;
-    pass_launches[3] = nrot > 0 ? 1 : 0;
+    for (int p = 0; p < 4; ++p) {
+        pass_ms[p] = tm.ms[p];
+        pass_launches[p] = tm.n[p];
+    }
     return rc;
 }
 
