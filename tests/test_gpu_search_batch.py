@@ -8,16 +8,11 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("mode,d", [("VecProduct", 48), ("prob", 48), ("Laplacian", 36), ("CC", 36), ("CC", 21),
-                                    ("VecProduct", 16)])
-@pytest.mark.parametrize("room", ["full", "least"])
-def test_profile_counts_the_launches_made(dev, mode, d, room):
+def _launches(dev, mode, d, n, nbytes):
+    """pass_launches of a search of n rotations in ``nbytes`` of scratch."""
     from vesper_python_gb300 import _native
     from vesper_python_gb300 import vesper as vg
-    n, code, prob = 500, vg.MODE_CODES[mode], mode == "prob"
-    per = (9 if prob else 4 if mode == "VecProduct" else 2) * d * d * (d // 2 + 1) * 8
-    base = min((64 << 20) // per, 2048)
-    nbytes = _native.size_query("vesper_search_workspace_size", d, code, 0 if room == "full" else base, n)
+    code, prob = vg.MODE_CODES[mode], mode == "prob"
     data, vec = torch.rand((d, d, d), dtype=torch.float64, device=dev.device), torch.rand((d, d, d, 3), device=dev.device)
     probs = torch.rand((4, d, d, d), device=dev.device) if prob else None
     spec = vg.target_spectra_device(data, vec, mode, 0.0, probs=probs, dev=dev)
@@ -29,6 +24,19 @@ def test_profile_counts_the_launches_made(dev, mode, d, room):
     p = lambda t: ctypes.c_void_p(t.data_ptr() if t is not None else None)  # noqa: E731
     _native.check(dev.lib.vesper_search_profile(p(spec), p(data), p(vec), p(probs), d, code, 0.0, p(mats), n, None, p(sc),
                                                 p(ln), 0, p(ws), nbytes, dev.stream, ms, nl, None))
+    return list(nl)
+
+
+@pytest.mark.parametrize("mode,d", [("VecProduct", 48), ("prob", 48), ("Laplacian", 36), ("CC", 36), ("CC", 21),
+                                    ("VecProduct", 16)])
+@pytest.mark.parametrize("room", ["full", "least"])
+def test_profile_counts_the_launches_made(dev, mode, d, room):
+    from vesper_python_gb300 import _native
+    from vesper_python_gb300 import vesper as vg
+    n, code, prob = 500, vg.MODE_CODES[mode], mode == "prob"
+    per = (9 if prob else 4 if mode == "VecProduct" else 2) * d * d * (d // 2 + 1) * 8
+    base = min((64 << 20) // per, 2048)
+    nbytes = _native.size_query("vesper_search_workspace_size", d, code, 0 if room == "full" else base, n)
     if vg.search_plan(d, mode, 0, 1, None, dev)[0] == 2:
         want = [1, 0, 0, 1]                                     # the fused kernel
     else:
@@ -36,4 +44,14 @@ def test_profile_counts_the_launches_made(dev, mode, d, room):
         full = max(base, min(n, 256, (1 << 30) // total))
         steps = -(-n // (full if room == "full" else base))
         want = [steps, steps, steps, 1]
-    assert list(nl) == want
+    assert _launches(dev, mode, d, n, nbytes) == want
+
+
+@pytest.mark.parametrize("mode,d,batch", [("VecProduct", 48, 101), ("prob", 48, 57), ("Laplacian", 36, 255), ("CC", 75, 26)])
+def test_default_batch_is_the_largest_that_fits(dev, mode, d, batch):
+    from vesper_python_gb300 import _native
+    from vesper_python_gb300 import vesper as vg
+    n = 4 * batch
+    nbytes = _native.size_query("vesper_search_workspace_size", d, vg.MODE_CODES[mode], batch, n)
+    assert _launches(dev, mode, d, n, nbytes) == [4, 4, 4, 1]
+    assert _launches(dev, mode, d, n, nbytes - 1) == [5, 5, 5, 1]
