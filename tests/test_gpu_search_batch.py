@@ -1,5 +1,6 @@
 """The batch that batch = 0 takes, by the launches that vesper_search_profile counts: the library's default
-where the workspace holds it, else the largest that the workspace holds."""
+where the workspace holds it, else the largest that the workspace holds; and search_device where the
+device has no room for the default."""
 import ctypes
 
 import pytest
@@ -55,3 +56,32 @@ def test_default_batch_is_the_largest_that_fits(dev, mode, d, batch):
     nbytes = _native.size_query("vesper_search_workspace_size", d, vg.MODE_CODES[mode], batch, n)
     assert _launches(dev, mode, d, n, nbytes) == [4, 4, 4, 1]
     assert _launches(dev, mode, d, n, nbytes - 1) == [5, 5, 5, 1]
+
+
+@pytest.mark.parametrize("mode,d", [("VecProduct", 48), ("prob", 36), ("Laplacian", 36), ("VecProduct", 16)])
+def test_search_device_with_little_memory(dev, monkeypatch, mode, d):
+    """The default batch's scratch is refused; a smaller batch gives the same bits.  A batch that the caller
+    names is not replaced."""
+    from vesper_python_gb300 import _native
+    from vesper_python_gb300 import vesper as vg
+    g = torch.Generator().manual_seed(d)
+    data = torch.rand((d, d, d), dtype=torch.float64, generator=g).to(dev.device)
+    vec, probs = torch.randn((d, d, d, 3), generator=g).to(dev.device), torch.rand((4, d, d, d), generator=g).to(dev.device)
+    kw = {"probs": probs} if mode == "prob" else {}
+    spec = vg.target_spectra_device(data, vec, mode, 0.0, dev=dev, **kw)
+    mats = dev.to_dev(vg.rot_matrices(vg.calc_angle_comb(30.0)[::5]))
+    n, code = int(mats.shape[0]), vg.MODE_CODES[mode]
+    ref = vg.search_device(spec, data, vec, mode, 0.0, mats, dev=dev, **kw)
+    for batch in (50, 9, 1):
+        room = _native.size_query("vesper_search_workspace_size", d, code, batch, n)
+
+        def workspace(key, nbytes):
+            if key[0] == "search" and nbytes > room:
+                raise torch.cuda.OutOfMemoryError("no room")
+            return torch.empty(nbytes, dtype=torch.uint8, device=dev.device)
+
+        monkeypatch.setattr(dev, "workspace", workspace)
+        got = vg.search_device(spec, data, vec, mode, 0.0, mats, dev=dev, **kw)
+        assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            vg.search_device(spec, data, vec, mode, 0.0, mats, batch=batch + 1, dev=dev, **kw)

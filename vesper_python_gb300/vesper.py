@@ -454,6 +454,26 @@ _SEARCH_SIZES = {}   # (device, side, mode, mixed, batch, rotations, options) ->
 #                      workspace tensor, options array)
 
 
+def _search_scratch(dev, d, code, batch, n, nbytes):
+    """(scratch of a search, its batch).  The library's default batch (0) asks
+    for up to 1 GiB; where the device has no room for that, a smaller batch,
+    whose results are the same."""
+    key = ("search", d, code, batch)
+    try:
+        return dev.workspace(key, nbytes), batch
+    except torch.cuda.OutOfMemoryError:
+        if batch > 0:
+            raise
+    for b in (128, 64, 32, 16, 8, 4, 2):
+        less = _native.size_query("vesper_search_workspace_size", d, code, b, n)
+        if less < nbytes:
+            try:
+                return dev.workspace(key, less), b
+            except torch.cuda.OutOfMemoryError:
+                pass
+    return dev.workspace(key, _native.size_query("vesper_search_workspace_size", d, code, 1, n)), 1
+
+
 def search_device(spec, data, vec, mode, ave, rotmats, probs=None, mix=None, batch=0, dev=None, profile=None,
                   opts=None, tuned=False, out=None):
     """vesper_search: (scores f32 [n][nscore], lin int32 [n][nscore]) CUDA tensors,
@@ -484,7 +504,7 @@ def search_device(spec, data, vec, mode, ave, rotmats, probs=None, mix=None, bat
         ent = _SEARCH_SIZES[sk] = (dev.lib.vesper_search_nscore(code, 1 if mix is not None else 0), ws_bytes,
                                    (ctypes.c_int * 3)(*[int(v) for v in opts]) if opts is not None else None)
     nscore, ws_bytes, copts = ent
-    ws = dev.workspace(("search", d, code, int(batch)), ws_bytes)
+    ws, batch = _search_scratch(dev, d, code, int(batch), max(n, 1), ws_bytes)
     if out is not None:
         scores, lin = out
         if (tuple(scores.shape) != (n, nscore) or tuple(lin.shape) != (n, nscore) or not scores.is_contiguous()
