@@ -8,7 +8,9 @@ library and raises if it cannot be loaded.
 from __future__ import annotations
 
 import ctypes
+import functools
 import glob
+import hashlib
 import os
 import shutil
 import subprocess
@@ -51,6 +53,17 @@ def _sources():
 
 def _deps():
     return _sources() + sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + [os.path.join(INCLUDE, "vesper_gb300.h")]
+
+
+@functools.lru_cache(maxsize=None)
+def source_digest() -> str:
+    """Names the library's sources: what was measured on one build is not taken
+    for another's."""
+    h = hashlib.sha1()
+    for p in _deps():
+        with open(p, "rb") as f:
+            h.update(f.read())
+    return h.hexdigest()[:12]
 
 
 def needs_build() -> bool:

@@ -12,7 +12,8 @@ and keeps the fastest (the register passes take only the batch; their other
 shapes are fixed per side).  The kernel family (register passes at sides 25 to
 100, radix-stage otherwise) is fixed by the side, so every candidate computes bit-identical results and the choice only changes speed.
 Results are cached per process and, unless VESPER_AUTOTUNE_CACHE is set to
-an empty string, in a JSON file (default ~/.cache/vesper_gb300/autotune.json).
+an empty string, in a JSON file (default ~/.cache/vesper_gb300/autotune.json),
+under the GPU's name and the library's sources: other kernels prefer other batches.
 """
 from __future__ import annotations
 
@@ -21,6 +22,8 @@ import os
 import threading
 
 import torch
+
+from . import _native
 
 _lock = threading.Lock()
 _mem: dict = {}
@@ -40,7 +43,7 @@ def _key(dim, mode, dev):
     name = _NAMES.get(dev.device)
     if name is None:
         name = _NAMES[dev.device] = torch.cuda.get_device_name(dev.device) if torch.cuda.is_available() else "cpu"
-    return f"{name}|d={dim}|mode={mode}"
+    return f"{name}|lib={_native.source_digest()}|d={dim}|mode={mode}"
 
 
 def _load_disk():
