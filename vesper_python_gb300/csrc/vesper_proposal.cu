@@ -1297,7 +1297,11 @@ extern "C" int vesper_prop_score(const float *ET, const float *EQ, int K, int d,
     if (!ET || !EQ || !rotmats || !scores || K < 1 || d < 1 || nrot < 0)
         return fail(VESPER_ERR_INVALID, "prop_score: bad args");
     if (nrot == 0) return VESPER_OK;
-    const size_t sm8 = score8_smem(d, 0);
+    // Fewer rotations than three blocks of the general kernel to an SM take one wave
+    // there (side 18, 304 rotations: 20.6 us, 26.8 staged; side 12 9.4 and 12.5); from
+    // 500 on the staged kernel is the faster one at most sides (18 29.0 and 26.9, 15
+    // 22.6 and 18.6, 12 10.4 and 14.4, at 800 16.1 and 14.1).
+    const size_t sm8 = nrot < 3 * kPropSMs ? 0 : score8_smem(d, 0);
     if (K == 8 && sm8) {
         // 4 rotations per thread once that leaves every SM a group of 16
         (nrot < 16 * kPropSMs ? score8<2> : score8<4>)(ET, EQ, d, rotmats, nrot, sm8, scores, (cudaStream_t)stream);
@@ -1475,7 +1479,12 @@ extern "C" int vesper_prop_score_bwd(const float *ET, const float *EQ, int K, in
     vesper_prop_score_bwd_workspace(K, d, &need);
     if (!workspace || workspace_bytes < need) return fail(VESPER_ERR_WORKSPACE, "prop_score_bwd: workspace");
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t sm8t = score8_smem(d, 0), sm8q = score8_smem(d, 1);
+    // Below side 9 few voxels share a rotation's staging and lists, and few of a block's
+    // threads own one: the general kernel up to side 6 (side 6, 24,624 rotations: 180
+    // us, 264 staged), at 7 and 8 for few rotations (side 7 24.9 and 28.8 at 304, 37.2
+    // and 34.9 at 1,008; side 8 20.8 and 22.9 at 152, 27.2 and 24.9 at 304).
+    const bool few = d <= 6 || (d <= 8 && nrot < (d == 7 ? 5 : 2) * kPropSMs);
+    const size_t sm8t = few ? 0 : score8_smem(d, 0), sm8q = score8_smem(d, 1);
     if (K == 8 && sm8t && sm8q) {
         // slots of the partial gradients (one per chunk of rotations), then the source
         // table of as many rotations as the workspace holds: groups of equal size
