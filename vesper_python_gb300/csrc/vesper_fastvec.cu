@@ -394,7 +394,11 @@ __global__ void __launch_bounds__(256) k_fvf_scan(const float *src, const FvGeom
 // entries of its band (most of a thresholded row is zero, and a zero adds nothing
 // to a pair sum).  The z axis's weight pairs are staged too when they fit (SW).
 // Every entry of the band for two rows per thread took 101 us (256^3 -> 42^3) and 30
-// (128^3 -> 28^3); now 41 and 9.5.
+// (128^3 -> 28^3); now 41 and 9.5.  Where the weights are not staged, two loads per entry
+// and sum cost more than the zeros once three tenths of a block's entries are not zero:
+// such blocks sum every entry of the band for two rows per thread, from one pair of
+// weight loads (256^3 -> 128^3, half of the voxels: 958 -> 663 us; zeros
+// are the same bits).
 constexpr int kZRows = 16;
 constexpr int kZThreads = 512;
 constexpr int kFfBatch = 8;    // band entries loaded per round by the y stage from global memory
@@ -415,6 +419,9 @@ __global__ void __launch_bounds__(kZThreads) k_fvf_z(const float *src, const FvG
     const int first = blockIdx.x * rows;
     const int nr = min(rows, t.count[0] - first);
     if (nr <= 0) return;   // block-uniform
+    __shared__ int total;  // non-zero entries of the block's rows
+    if (!SW && threadIdx.x == 0) total = 0;
+    if (!SW) __syncthreads();
     ZEntry *ent = (ZEntry *)smem;                                      // [rows][S2]
     unsigned short *cnt = (unsigned short *)(ent + rows * S2);         // [rows][CN]
     float2 *sw = (float2 *)(smem + fvf_z_rows_smem(S2, rows));         // [WB][d] when SW
@@ -440,10 +447,46 @@ __global__ void __launch_bounds__(kZThreads) k_fvf_z(const float *src, const FvG
             n += __popc(m);
         }
         if (lane == 0) cnt[r * CN + S2] = (unsigned short)n;
+        if (!SW && lane == 0) atomicAdd(&total, n);
     }
     __syncthreads();
     const int *stp = t.stp + 2 * d, *len = t.len + 2 * d;
     const float2 *w = SW ? sw : gw, *wp = SW ? swp : gwp;
+    if (!SW && total > nr * S2 * 3 / 10) {   // dense rows: every entry, two rows per thread
+        float *full = (float *)smem;         // [nr + 1][S2], the last row zero
+        __syncthreads();
+        for (int e = threadIdx.x; e < (nr + 1) * S2; e += kZThreads) {
+            const int r = e / S2;
+            full[e] = r < nr ? __ldg(src + (size_t)t.list[first + r] * S2 + (e - r * S2)) : 0.f;
+        }
+        __syncthreads();
+        for (int it = threadIdx.x; it < (nr + 1) / 2 * d; it += kZThreads) {
+            const int r = it / d * 2, z = it - r / 2 * d, n = len[z];
+            const float *v0 = full + r * S2 + stp[z], *v1 = v0 + S2;
+            float s0h[2] = {}, s0l[2] = {}, s1h[2] = {}, s1l[2] = {};
+#pragma unroll 2
+            for (int k = 0; k < n; ++k) {
+                const float2 a = __ldg(w + (size_t)k * d + z), b = __ldg(wp + (size_t)k * d + z);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const float v = (u ? v1 : v0)[k];
+                    float ph, pl;
+                    ff_mul_f(a.x, a.y, v, ph, pl);
+                    ff_add(s0h[u], s0l[u], ph, pl);
+                    ff_mul_f(b.x, b.y, v, ph, pl);
+                    ff_add(s1h[u], s1l[u], ph, pl);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (r + u < nr) {
+                    const size_t o = (size_t)t.list[first + r + u] * d + z;
+                    A0[o] = make_float2(s0h[u], s0l[u]);
+                    A1[o] = make_float2(s1h[u], s1l[u]);
+                }
+        }
+        return;
+    }
     for (int it = threadIdx.x; it < nr * d; it += kZThreads) {
         const int r = it / d, z = it - r * d, s = min(stp[z], S2), n = len[z];
         const int lo = cnt[r * CN + s], hi = n > 0 ? cnt[r * CN + s + n] : lo;
@@ -575,18 +618,93 @@ __global__ void __launch_bounds__(kYThreads) k_fvf_y(const FvGeom g, const AxisT
     }
 }
 
+// The finish of voxel v from its sums D, Px, Py, Pz (VESPER_1_prob_new.py:242-255).
+__device__ __forceinline__ void fvf_finish(const AxisTables &t, int d, int v, float2 sd, float2 sx, float2 sy, float2 sz,
+                                           double *data_out, float *data_f32, float *vec_out) {
+    const int x = v / (d * d), yz = v - x * d * d, y = yz / d, z = yz - y * d;
+    const double dt = (double)sd.x + (double)sd.y;
+    float o0 = 0.f, o1 = 0.f, o2 = 0.f;
+    if (dt != 0.0) {
+        const double px = (double)sx.x + (double)sx.y, py = (double)sy.x + (double)sy.y, pz = (double)sz.x + (double)sz.y;
+        const double rd = __ddiv_rn(1.0, dt);
+        const double t0 = __dsub_rn(__dmul_rn(px, rd), t.pos[x]);
+        const double t1 = __dsub_rn(__dmul_rn(py, rd), t.pos[d + y]);
+        const double t2 = __dsub_rn(__dmul_rn(pz, rd), t.pos[2 * d + z]);
+        double dv = __dadd_rn(__dmul_rn(t0, t0), __dmul_rn(t1, t1));
+        dv = __dsqrt_rn(__dadd_rn(dv, __dmul_rn(t2, t2)));
+        if (dv == 0.0) dv = 1.0;
+        const double rdv = __ddiv_rn(1.0, dv);
+        o0 = (float)__dmul_rn(t0, rdv);
+        o1 = (float)__dmul_rn(t1, rdv);
+        o2 = (float)__dmul_rn(t2, rdv);
+    }
+    data_out[v] = dt;
+    if (data_f32) data_f32[v] = (float)dt;
+    vec_out[3 * (size_t)v + 0] = o0;
+    vec_out[3 * (size_t)v + 1] = o1;
+    vec_out[3 * (size_t)v + 2] = o2;
+}
+
 // stage 3 (x) and the finish, four lanes per listed voxel, one for each of its sums
 // D, Px, Py, Pz: the column's sums are read along x between the first and last plane
 // with a non-zero value, kXBatch entries in flight.  Blocks over all voxels, a slab of
 // B0, B1 and B2 in shared memory and 9 of 32 lanes at work took 34 us for 256^3 -> 42^3.
 // With the stages above the whole call went from 233 to 121 us there and from 73 to 59
 // for 128^3 -> 28^3.
+// MANY (grids of kXGrid voxels and more): from kXMany listed voxels on, about 16 warps of
+// them per SM, a thread has a voxel and its four sums: a warp's loads then are whole
+// lines, and the sums share them (200^3 -> 75^3, every voxel: 172 -> 105 us, a ball 54 ->
+// 40).  Smaller grids keep the form for few voxels alone, which is faster without the
+// other's registers (100^3 -> 50^3, a ball: 12 us, 15 with them).
+constexpr int kXMany = 80000;
+constexpr size_t kXGrid = 150000;
+constexpr int kXBatch1 = 4;
+template <bool MANY>
 __global__ void __launch_bounds__(128) k_fvf_x(const FvGeom g, const AxisTables t, const float2 *B0, const float2 *B1,
                                                const float2 *B2, double *data_out, float *data_f32, float *vec_out) {
-    const int i = blockIdx.x * 32 + (threadIdx.x >> 2), q = threadIdx.x & 3, d = g.d, nv = t.count[1];
+    const int d = g.d, nv = t.count[1];
+    const size_t plane = (size_t)d * d;
+    if (MANY && nv >= kXMany) {
+        const int i = blockIdx.x * 128 + threadIdx.x;
+        if (i >= nv) return;
+        const int v = t.voxels[i], x = v / (d * d), yz = v - x * d * d;
+        const int s = t.stp[x], k0 = max(0, t.count[2] - s), n = min(t.len[x], t.count[3] + 1 - s);
+        const float2 *w = t.wf + x, *wp = t.wpf + x;
+        const size_t o = (size_t)s * plane + yz;
+        float2 sum[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sum[q] = make_float2(0.f, 0.f);
+        for (int k = k0; k < n; k += kXBatch1) {
+            float2 wx[kXBatch1], wxp[kXBatch1], b0[kXBatch1], b1[kXBatch1], b2[kXBatch1];
+#pragma unroll
+            for (int u = 0; u < kXBatch1; ++u) {
+                const int e = min(k + u, n - 1);
+                wx[u] = __ldg(w + (size_t)e * d);
+                wxp[u] = __ldg(wp + (size_t)e * d);
+                b0[u] = __ldg(B0 + o + e * plane);
+                b1[u] = __ldg(B1 + o + e * plane);
+                b2[u] = __ldg(B2 + o + e * plane);
+                if (k + u >= n) b0[u] = b1[u] = b2[u] = make_float2(0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < kXBatch1; ++u) {
+                float ph, pl;
+                ff_mul(b0[u], wx[u], ph, pl);
+                ff_add(sum[0].x, sum[0].y, ph, pl);
+                ff_mul(b0[u], wxp[u], ph, pl);
+                ff_add(sum[1].x, sum[1].y, ph, pl);
+                ff_mul(b1[u], wx[u], ph, pl);
+                ff_add(sum[2].x, sum[2].y, ph, pl);
+                ff_mul(b2[u], wx[u], ph, pl);
+                ff_add(sum[3].x, sum[3].y, ph, pl);
+            }
+        }
+        fvf_finish(t, d, v, sum[0], sum[1], sum[2], sum[3], data_out, data_f32, vec_out);
+        return;
+    }
+    const int i = blockIdx.x * 32 + (threadIdx.x >> 2), q = threadIdx.x & 3;
     if (blockIdx.x * 32 >= nv) return;
     const int vi = t.voxels[min(i, nv - 1)], xi = vi / (d * d);
-    const size_t plane = (size_t)d * d;
     const int s = t.stp[xi], k0 = max(0, t.count[2] - s), n = min(t.len[xi], t.count[3] + 1 - s);
     const float2 *w = (q == 1 ? t.wpf : t.wf) + xi, *b = (q < 2 ? B0 : q == 2 ? B1 : B2) + (size_t)s * plane + vi % (d * d);
     float sh = 0.f, sl = 0.f;
@@ -612,30 +730,8 @@ __global__ void __launch_bounds__(128) k_fvf_x(const FvGeom g, const AxisTables 
     __syncthreads();
     const int f = blockIdx.x * 32 + threadIdx.x;
     if (threadIdx.x >= 32 || f >= nv) return;
-    const int v = t.voxels[f], x = v / (d * d), yz = v - x * d * d, y = yz / d, z = yz - y * d;
-    const float2 sd = sums[0][threadIdx.x], sx = sums[1][threadIdx.x], sy = sums[2][threadIdx.x], sz = sums[3][threadIdx.x];
-    const double dt = (double)sd.x + (double)sd.y;
-    float o0 = 0.f, o1 = 0.f, o2 = 0.f;
-    if (dt != 0.0) {
-        // VESPER_1_prob_new.py:242-255
-        const double px = (double)sx.x + (double)sx.y, py = (double)sy.x + (double)sy.y, pz = (double)sz.x + (double)sz.y;
-        const double rd = __ddiv_rn(1.0, dt);
-        const double t0 = __dsub_rn(__dmul_rn(px, rd), t.pos[x]);
-        const double t1 = __dsub_rn(__dmul_rn(py, rd), t.pos[d + y]);
-        const double t2 = __dsub_rn(__dmul_rn(pz, rd), t.pos[2 * d + z]);
-        double dv = __dadd_rn(__dmul_rn(t0, t0), __dmul_rn(t1, t1));
-        dv = __dsqrt_rn(__dadd_rn(dv, __dmul_rn(t2, t2)));
-        if (dv == 0.0) dv = 1.0;
-        const double rdv = __ddiv_rn(1.0, dv);
-        o0 = (float)__dmul_rn(t0, rdv);
-        o1 = (float)__dmul_rn(t1, rdv);
-        o2 = (float)__dmul_rn(t2, rdv);
-    }
-    data_out[v] = dt;
-    if (data_f32) data_f32[v] = (float)dt;
-    vec_out[3 * (size_t)v + 0] = o0;
-    vec_out[3 * (size_t)v + 1] = o1;
-    vec_out[3 * (size_t)v + 2] = o2;
+    fvf_finish(t, d, t.voxels[f], sums[0][threadIdx.x], sums[1][threadIdx.x], sums[2][threadIdx.x], sums[3][threadIdx.x],
+               data_out, data_f32, vec_out);
 }
 
 // smallest band weight of the geometry (|r| <= fmaxd + 1 on each axis)
@@ -764,7 +860,8 @@ extern "C" int vesper_fastvec(const float *src, int sx, int sy, int sz, double s
         float2 *b0 = reinterpret_cast<float2 *>(B0), *b1 = reinterpret_cast<float2 *>(B1),
                *b2 = reinterpret_cast<float2 *>(B2);
         const unsigned row_blocks = (unsigned)std::min<size_t>((nrows + 63) / 64, 1 << 14);
-        const unsigned vox_blocks = (unsigned)(((size_t)dim * dim * dim + 255) / 256);
+        const size_t vox = (size_t)dim * dim * dim;
+        const unsigned vox_blocks = (unsigned)((vox + 255) / 256);
         if (sz % 4 == 0 && ((uintptr_t)src & 15) == 0)
             k_fvf_scan<true><<<row_blocks + vox_blocks, 256, 0, st>>>(src, g, t, (int)row_blocks, data_out, data_f32, vec_out);
         else
@@ -791,8 +888,8 @@ extern "C" int vesper_fastvec(const float *src, int sx, int sy, int sz, double s
         allow_smem(k_fvf_y, sy2);
         k_fvf_y<<<dim3(nt, sx, (unsigned)((dim + yc - 1) / yc)), kYThreads, sy2, st>>>(g, t, zw, yc, ry, a0, a1, b0, b1, b2);
         VG_CHECK_LAUNCH("k_fvf_y");
-        k_fvf_x<<<(unsigned)(((size_t)dim * dim * dim + 31) / 32), 128, 0, st>>>(g, t, b0, b1, b2, data_out, data_f32,
-                                                                                   vec_out);
+        (vox >= kXGrid ? k_fvf_x<true> : k_fvf_x<false>)
+            <<<(unsigned)((vox + 31) / 32), 128, 0, st>>>(g, t, b0, b1, b2, data_out, data_f32, vec_out);
         VG_CHECK_LAUNCH("k_fvf_x");
         return VESPER_OK;
     }
