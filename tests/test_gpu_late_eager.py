@@ -72,3 +72,27 @@ def test_eager_proposal_refinement_equals_host_driven(dev, fallback):
                 assert (tuple(x.angle), tuple(x.vec_trans), x.vec_score, x.overlap, x.cc, x.pcc, x.dot_score) == \
                     (tuple(y.angle), tuple(y.vec_trans), y.vec_score, y.overlap, y.cc, y.pcc, y.dot_score)
                 assert np.array_equal(x.translation, y.translation)
+
+
+@pytest.mark.parametrize("mode", ["VecProduct", "Overlap", "Laplacian"])
+def test_graph_refinement_equals_host_driven(dev, mode):
+    """The captured form against the host-driven refinement: at these sides the eager form runs the captured
+    form's own stage on the same side streams."""
+    from vesper_python_gb300 import align, synth
+    items = []
+    for i in range(9):
+        pair = synth.make_pair(80 + i, 48 + 16 * (i % 3), 40, 14.0 + 4 * (i % 3))
+        items.append((dev.to_dev(pair.map1), dev.to_dev(pair.map2), 1.0, 1.0, pair.orig1, pair.orig2))
+    p = align.AlignParams(t=0.1, T=0.1, s=3.0, A=30.0, N=10, mode=mode)
+    host = align.Aligner(dev)
+    host.LATE_SIDE = 0
+    ref = host.align_many(items, p)
+    al = align.Aligner(dev)
+    for _ in range(2):
+        al.pair_events = []
+        for a, b in zip(al.align_many(items, p, graph=True), ref):
+            assert (a.dim, a.std, a.ave, a.top) == (b.dim, b.std, b.ave, b.top)
+            assert [(tuple(x.angle), tuple(x.vec_trans), x.vec_score, x.overlap, x.cc, x.pcc, x.dot_score)
+                    for x in a.models] == \
+                [(tuple(x.angle), tuple(x.vec_trans), x.vec_score, x.overlap, x.cc, x.pcc, x.dot_score) for x in b.models]
+        assert len(al.pair_events) == 9

@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(128) k_conv_s(const float *in, const float *ma
     const int split = SPL > 1 ? threadIdx.x / (128 / SPL) : 0;
     const int u = blockIdx.x * (128 / SPL) + (SPL > 1 ? threadIdx.x % (128 / SPL) : threadIdx.x);
     if (SPL == 1 && u >= d * d * nzs) return;
-    const int x = u / (d * nzs), y = (u / nzs) % d, z0 = (u % nzs) * ZS;   // x >= d past the end: no row is on the grid
+    const int x = u / (d * nzs), y = (u / nzs) % d, z0 = (u % nzs) * ZS;   // x >= d past the end: each row is tested, nothing is stored
     // the 9 rows' places and the z values on the grid, a bit each
     unsigned rows = 0u, zs = 0u;
 #pragma unroll
