@@ -76,10 +76,10 @@ MODE_NAMES = {"V": "VecProduct", "O": "Overlap", "C": "CC", "P": "PCC", "L": "La
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per rotation of the
 # dominant search kernel (search pass A), mode V, by grid side, from ncu
-# captures of ``bench.py --case search<d> <nrot> <batch>`` at the batches the
-# workloads run (256 rotations per launch at sides 28-32, 128 at 75), caches
-# left as the previous launches leave them (profiles/search_pass_a_dram.md).
-PASS_A_DRAM_PER_ROT = {28: 264845, 30: 266378, 32: 290951, 75: 4726406}
+# captures of ``bench.py --case search<d> <nrot> <batch>`` at the batch the
+# workloads run (256 rotations per launch), caches left as the previous
+# launches leave them (profiles/search_pass_a_dram.md).
+PASS_A_DRAM_PER_ROT = {28: 251575, 30: 265569, 32: 292045, 75: 4934569}
 
 
 def parse():

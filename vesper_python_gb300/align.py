@@ -301,11 +301,14 @@ class Aligner:
             stats, sh = self._global_stage(P, p, mats, nang)
         # the refinement and rescoring from the device's own results: in the graph form
         # always, in eager calls where every grid is small.  It searches all N x 27
-        # slots of a pair, about 120 rotations more than the distinct ones, and lets the
-        # pairs' chains of short launches overlap, with no host round trip between the
-        # stages (16 pairs of sides 28 to 32: refinement and rescoring 6.3 -> 2.2 ms,
-        # the whole call 19.9 -> 15.0); at larger sides the 120 rotations cost more than
-        # that gives.
+        # slots of a pair, about 120 rotations more than the distinct ones at N = 10, and
+        # lets the pairs' chains of short launches overlap, with no host round trip
+        # between the stages and no host arithmetic (whole calls, host-driven -> this: 16
+        # pairs of sides 30 to 32 with the proposal 19.5 -> 14.7 ms; without, sides 26 to
+        # 30, N = 10 15.0 -> 10.7, N = 300 91 -> 66).  The line at side 32 is a cautious
+        # one: up to side 60 it was the faster form too (16 pairs of sides 40 to 45 34.0
+        # -> 30.4 ms, of 52 to 60 68.9 -> 65.5), from about 70 on the slots cost more
+        # than that gives where N is 100 (sides 70 to 77 418 and 433).
         late_eager = not graph and max(st.dim for st in P) <= self.LATE_SIDE
         device_late = (graph or late_eager) and mode not in ("PCC", "CC") and p.A > 5.0 and self.group is None and \
             self._grid_rows(p.A, angle_comb) is not None

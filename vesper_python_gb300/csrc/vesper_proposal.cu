@@ -62,7 +62,10 @@ __device__ __forceinline__ int quot(int v, int d, unsigned m) { return d == 1 ? 
 // of one per row behind its bounds test (the four layers of two side-15 maps 490 -> 150
 // us, of 16 maps 460 -> 290).  Sums in the order of k_conv_fwd (bias, then channel,
 // then tap) and of k_conv_bwd_data (channel, then tap); a tap off the grid adds +-0, so
-// results are the same bits for finite weights.
+// results are the same bits for finite weights.  (One that is not finite gives NaN at the
+// border, where k_conv_fwd has none.  Blocks that test their weights and take a loop of
+// their own were measured: the registers of either form cost 32 -> 32 channels, 16 maps
+// of side 15, 119 -> 130 to 152 us.)
 // BWD: the sums run over the layer's output channels (their gradient masked where a
 // ReLU let nothing through) and the taps are mirrored.
 // SPL: a block's warps share 32 threads' voxels and sum nin / SPL channels each (added

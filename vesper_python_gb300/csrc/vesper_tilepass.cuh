@@ -17,19 +17,19 @@
 // steps in the opposite order.
 //
 // What bounds them (GB300, mode V, microseconds per rotation A / B / C, against
-// the kernels they replace): side 75 2.50 / 1.52 / 0.87 (one block-wide step after
-// another, general gather in line: 5.41 / 1.74 / 1.04), side 48 0.67 / 0.66 / 0.29
-// (radix stages 2.26 / 1.60 / 1.06), side 80 2.72 / 2.4 / 1.12 (11.9 / 7.4 / 3.1),
-// prob mode at side 64 3.3 / 2.6 / 1.16 (18.0 / 5.4 / 2.7).  A is bound by issue
-// slots and shared-memory wavefronts together (56 % and 58 % at 15 warps per SM;
-// one warp per tile gives 30): strides without bank conflicts took side 75 from
-// 4.17 to 3.93, one warp per tile within 64 registers to 3.48, and the middle
+// the kernels they replace): side 75 2.57 / 1.56 / 0.91 (one block-wide step after
+// another, general gather in line: 5.41 / 1.74 / 1.04), side 48 0.69 / 0.60 / 0.29
+// (radix stages 2.26 / 1.60 / 1.06), side 80 2.82 / 2.20 / 1.16 (11.9 / 7.4 / 3.1),
+// prob mode at side 64 3.4 / 2.6 / 1.17 (18.0 / 5.4 / 2.7).  A is bound by issue
+// slots and the L1 data path together (68 % and 72 % at side 75, 73 % and 83 % at 48;
+// one warp per tile gives 45 % of the warps): strides without bank conflicts took side
+// 75 from 4.17 to 3.93, one warp per tile within 64 registers to 3.48, and the middle
 // voxels of odd sides, loaded together and shared out over the CTA, to 3.14; prob mode
 // at side 64 4.51 -> 3.97 with lines and columns that do not meet in a bank.  A query
 // fills a ball of its grid, and the rotated one a ball too: leaving out the z steps,
 // lines and planes outside it took side 75 from 3.14 to 2.50 and prob mode at side 64
 // from 3.97 to 3.30 (a ball of 0.42 of the side).  C is bound
-// by issue slots (75 %): one 32-bit comparison per voxel instead of a 64-bit key took
+// by issue slots (72 %): one 32-bit comparison per voxel instead of a 64-bit key took
 // side 75 from 0.98 to 0.87.  B is
 // bound by the S and T it reads: T from L2 once per 8 rotations instead of once
 // each took side 75 from 1.74 to 1.52.
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(ta_warps<N1, N2>() * 32, ta_ctas<kSrcProb, N1,
 // the cubes; a shape other than a thread per item of the second forward step is taken
 // where that promises a tenth (a sixth for one channel, whose three rotations already
 // share the barriers: below that 42 and 100 lost), and never for PFA sides, which have
-// no fourth step (side 75: 1.61 either way).  Microseconds per rotation, a thread per
+// no fourth step (side 75: 1.5 to 1.6 either way).  Microseconds per rotation, a thread per
 // item before and after: mode V 48 0.69 -> 0.61, 54 1.18 -> 0.94, 72 4.19 -> 2.33,
 // 81 5.57 -> 3.16, 88 5.89 -> 3.88, 91 6.81 -> 4.37, 96 9.08 -> 6.30; one channel 39
 // 0.27 -> 0.18, 66 0.96 -> 0.65, 78 2.44 -> 1.13, 96 4.01 -> 2.01; prob mode 48 1.65 ->
