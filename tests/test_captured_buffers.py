@@ -62,12 +62,30 @@ def test_scratch_without_a_capture_is_given_back_and_kept_scratch_is_bounded(mon
         assert sum(t.numel() for t in dev._kept) <= buf.numel() < 2 * nbytes + 8000
 
 
+def test_aligners_do_not_share_scratch(monkeypatch):
+    """Graphs of two aligners are captured on the same capture stream and may be replayed side by side."""
+    dev, state = _device(monkeypatch)
+    dev.lib = None
+    state["capturing"] = True
+    users = [align.Aligner(dev), align.Aligner(dev)]
+    spans = []
+    for d in [dev] + [al.dev for al in users]:
+        buf = d.workspace(("search", 28, 0, 0), 4096)
+        assert buf is d.workspace(("search", 28, 0, 0), 4000)
+        spans.append((buf.data_ptr(), buf.data_ptr() + buf.numel()))
+    spans.sort()
+    assert all(a[1] <= b[0] for a, b in zip(spans, spans[1:]))
+    assert all(al.dev.device == dev.device and al.dev.lib is dev.lib for al in users)
+
+
 def test_captured_stage_keeps_the_networks_weights(monkeypatch):
     """Other weights, of the same network or of one that takes its place, are another signature, and the weights
     that a captured stage reads are not given back."""
     monkeypatch.setattr(torch.cuda, "CUDAGraph", lambda: types.SimpleNamespace(replay=lambda: None))
     monkeypatch.setattr(torch.cuda, "graph", lambda g: contextlib.nullcontext())
-    al = align.Aligner(types.SimpleNamespace(lib=None))
+    dev, _ = _device(monkeypatch)
+    dev.lib = None
+    al = align.Aligner(dev)
     monkeypatch.setattr(al, "_global_stage", lambda P, p, mats, nang: (None, None))
     m = torch.zeros(4, 4, 4)
     st = align._Pair(m, m, 1.0, 1.0, np.zeros(3), np.zeros(3))

@@ -178,7 +178,7 @@ class Aligner:
     """Holds the device, cached angle-grid matrices and scratch buffers."""
 
     def __init__(self, dev: vg.Device | None = None, group=None):
-        self.dev = dev or vg.default_device()
+        self.dev = (dev or vg.default_device()).with_own_scratch()
         # torch.distributed process group: with one, every search splits its
         # rotations across the group's ranks (one GPU each) and gathers the
         # per-rotation results (vg.search_device_sharded); the CUDA-graph form

@@ -94,6 +94,14 @@ class Device:
             self._captured.add(key)
         return buf
 
+    def with_own_scratch(self):
+        """The same device with scratch of its own.  Streams keep the scratch of
+        eager calls apart; captures share one capture stream, so owners whose
+        graphs may be replayed at the same time each need theirs."""
+        d = copy.copy(self)
+        d._ws, d._captured, d._kept = {}, set(), []
+        return d
+
     def to_dev_async(self, a):
         """Small host array -> device without waiting on the stream: staged in
         pinned memory (torch's caching host allocator keeps the staging block
