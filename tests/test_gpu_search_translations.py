@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 MIX = (0.5, 0.7, 0.1, 0.3, 0.2)   # alpha, vstd, vave, pstd, pave
 
 
-@pytest.mark.parametrize("mode,d", [(m, d) for m in ("VecProduct", "prob", "CC", "PCC", "Laplacian") for d in PFA[m]])
+@pytest.mark.parametrize("mode,d", [("VecProduct", 13)] +
+                         [(m, d) for m in ("VecProduct", "prob", "CC", "PCC", "Laplacian") for d in PFA[m]])
 def test_split_sides_find_the_largest_score(dev, mode, d):
     from vesper_python_gb300 import vesper as vg
     rng = np.random.default_rng(d)
