@@ -252,10 +252,10 @@ __global__ void k_conv_bwd_weight(const float *dout, const float *out, int relu,
 // sits in shared memory with a zero border, so a voxel's 27 neighbours are plain
 // loads, each used for kWgCo products, where one block per (co, ci) pair spent its
 // instructions on the neighbours' bounds (the eight layers of a training step at side 15
-// 354 -> 247 us).  2 channels and 256 threads: 4 channels take 192 registers.
+// 354 -> 237 us).  2 channels and 256 threads: 4 channels take 192 registers.
 // The products with the border and with zero gradients, which k_conv_bwd_weight leaves
-// out, add zeros: the same sums for finite values.  A block that meets another value
-// sums again without them.
+// out, add zeros: the same sums for finite values.  A block whose sums are not finite
+// makes them again without.
 constexpr int kWgCo = 2;
 constexpr int kWgThreads = 256;
 __global__ void __launch_bounds__(kWgThreads) k_conv_bwd_weight_s(const float *dout, const float *out, int relu,
@@ -266,12 +266,10 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_bwd_weight_s(const float *d
     const int n = d * d * d, p = d + 2;
     const int ci = blockIdx.x % cin, co0 = blockIdx.x / cin * kWgCo;
     const float *src = in + (size_t)ci * n;
-    bool odd = false;   // a value that is not finite
     for (int e = threadIdx.x; e < p * p * p; e += kWgThreads) {
         const int q = quot(e, p, mp), x = quot(q, p, mp) - 1, y = q - (x + 1) * p - 1, z = e - q * p - 1;
         const bool on = x >= 0 && y >= 0 && z >= 0 && x < d && y < d && z < d;
         pad[e] = on ? __ldg(src + (x * d + y) * d + z) : 0.f;
-        odd |= !(fabsf(pad[e]) <= FLT_MAX);
     }
     __syncthreads();
     float acc[kWgCo][28];
@@ -279,6 +277,7 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_bwd_weight_s(const float *d
     for (int j = 0; j < kWgCo; ++j)
 #pragma unroll
         for (int o = 0; o < 28; ++o) acc[j][o] = 0.f;
+#pragma unroll 4
     for (int v = threadIdx.x; v < n; v += kWgThreads) {
         float g[kWgCo];
 #pragma unroll
@@ -287,7 +286,6 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_bwd_weight_s(const float *d
             g[j] = __ldg(dout + i);
             if (relu && !(__ldg(out + i) > 0.f)) g[j] = 0.f;
             acc[j][27] += g[j];
-            odd |= !(fabsf(g[j]) <= FLT_MAX);
         }
         const int q = quot(v, d, md), x = quot(q, d, md);
         const float *c = pad + (x * p + q - x * d) * p + v - q * d;
@@ -296,35 +294,6 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_bwd_weight_s(const float *d
             const float t = c[(o / 9 * p + o / 3 % 3) * p + o % 3];
 #pragma unroll
             for (int j = 0; j < kWgCo; ++j) acc[j][o] = fmaf(g[j], t, acc[j][o]);
-        }
-    }
-    if (__syncthreads_or(odd)) {
-        // once more, without the products that k_conv_bwd_weight leaves out: of a zero
-        // gradient, and with a neighbour off the grid
-#pragma unroll 1
-        for (int j = 0; j < kWgCo; ++j) {
-            float a[28];
-#pragma unroll
-            for (int o = 0; o < 28; ++o) a[o] = 0.f;
-#pragma unroll 1
-            for (int v = threadIdx.x; v < n; v += kWgThreads) {
-                const size_t i = (size_t)(co0 + j) * n + v;
-                const float g = relu && !(__ldg(out + i) > 0.f) ? 0.f : __ldg(dout + i);
-                if (g == 0.f) continue;
-                const int x = v / (d * d), y = v / d % d, z = v % d;
-#pragma unroll
-                for (int o = 0; o < 27; ++o) {
-                    const int xx = x + o / 9, yy = y + o / 3 % 3, zz = z + o % 3;   // in pad
-                    if (xx < 1 || yy < 1 || zz < 1 || xx > d || yy > d || zz > d) continue;
-                    a[o] = fmaf(g, pad[(xx * p + yy) * p + zz], a[o]);
-                }
-                a[27] += g;
-            }
-#pragma unroll
-            for (int k = 0; k < kWgCo; ++k)
-#pragma unroll
-                for (int o = 0; o < 28; ++o)
-                    if (k == j) acc[k][o] = a[o];
         }
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -337,15 +306,43 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_bwd_weight_s(const float *d
             if (lane == 0) red[warp][j * 28 + o] = t;
         }
     __syncthreads();
-    for (int e = threadIdx.x; e < kWgCo * 28; e += kWgThreads) {
+    const int e = threadIdx.x;
+    auto total = [&]() {
         float t = 0.f;
-        for (int w = 0; w < kWgThreads / 32; ++w) t += red[w][e];
-        const int j = e / 28, o = e % 28;
-        if (o < 27)
-            dW[((size_t)(co0 + j) * cin + ci) * 27 + o] += t;
-        else if (ci == 0)
-            db[co0 + j] += t;
+        if (e < kWgCo * 28)
+            for (int w = 0; w < kWgThreads / 32; ++w) t += red[w][e];
+        return t;
+    };
+    float t = total();
+    if (__syncthreads_or(!(fabsf(t) <= FLT_MAX))) {
+        // once more, one sum after another, without the products that k_conv_bwd_weight
+        // leaves out: of a zero gradient, and off the grid
+#pragma unroll 1
+        for (int f = 0; f < kWgCo * 28; ++f) {
+            const int o = f % 28, ox = o / 9, oy = o / 3 % 3, oz = o % 3;
+            float a = 0.f;
+#pragma unroll 1
+            for (int v = threadIdx.x; v < n; v += kWgThreads) {
+                const size_t i = (size_t)(co0 + f / 28) * n + v;
+                const float g = relu && !(__ldg(out + i) > 0.f) ? 0.f : __ldg(dout + i);
+                const int x = v / (d * d) + ox, y = v / d % d + oy, z = v % d + oz;   // in pad
+                if (o == 27)
+                    a += g;
+                else if (g != 0.f && x >= 1 && y >= 1 && z >= 1 && x <= d && y <= d && z <= d)
+                    a = fmaf(g, pad[(x * p + y) * p + z], a);
+            }
+            for (int k = 16; k > 0; k >>= 1) a += __shfl_down_sync(0xffffffffu, a, k);
+            if (lane == 0) red[warp][f] = a;
+        }
+        __syncthreads();
+        t = total();
     }
+    if (e >= kWgCo * 28) return;
+    const int j = e / 28, o = e % 28;
+    if (o < 27)
+        dW[((size_t)(co0 + j) * cin + ci) * 27 + o] += t;
+    else if (ci == 0)
+        db[co0 + j] += t;
 }
 
 // ---- network input ---------------------------------------------------------------
