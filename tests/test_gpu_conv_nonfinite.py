@@ -55,3 +55,33 @@ def test_weight_gradient(dev, d, where):
         _same(both[k], torch.cat([o[k] for o in one]))
     if where == "masked":
         assert torch.equal(both[0], torch.ones_like(both[0]))
+
+
+@pytest.mark.parametrize("d", [1, 3, 8, 13])
+@pytest.mark.parametrize("nmap", [1, 40])     # one voxel per thread, and four
+@pytest.mark.parametrize("relu", [0, 1])
+@pytest.mark.parametrize("where", ["weights", "input", "both", "bias"])
+def test_forward(dev, d, nmap, relu, where):
+    """Four output channels per thread against one (a channel count that four does not divide)."""
+    from vesper_python_gb300 import _native
+    g = torch.Generator().manual_seed(d)
+    cin = 5
+    x, W, b = _whole(g, nmap, cin, d, d, d), _whole(g, 8, cin, 27), _whole(g, 8)
+    if where in ("weights", "both"):
+        W[0, 0, 0], W[1, 2, 14], W[2, 4, 26], W[5, 1, 3] = INF, -INF, NAN, INF
+    if where in ("input", "both"):
+        x[0, 1, d // 2, 0, d - 1], x[-1, 3, 0, d // 2, 0] = INF, NAN
+    if where == "bias":
+        b[1], b[6] = INF, NAN
+    x, W, b = x.to(dev.device), W.to(torch.bfloat16).to(dev.device), b.to(dev.device)
+
+    def layer(lo, hi):
+        o = torch.full((nmap, hi - lo, d, d, d), 7.0, device=dev.device)
+        _native.check(dev.lib.vesper_prop_conv_fwd(_p(x), cin, _p(W[lo:hi].contiguous()), _p(b[lo:hi].contiguous()), hi - lo,
+                                                   d, relu, nmap, _p(o), dev.stream))
+        return o
+
+    fast, plain = layer(0, 8), torch.cat([layer(i, i + 1) for i in range(8)], 1)
+    assert torch.equal(fast.isnan(), plain.isnan())
+    assert torch.equal(torch.nan_to_num(fast, nan=0.0, posinf=9e9, neginf=-9e9),
+                       torch.nan_to_num(plain, nan=0.0, posinf=9e9, neginf=-9e9))

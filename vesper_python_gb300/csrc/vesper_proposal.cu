@@ -54,6 +54,25 @@ __global__ void k_conv_fwd(const float *in, int cin, const __nv_bfloat16 *W, con
 __host__ __device__ __forceinline__ unsigned recip(unsigned d) { return 0xffffffffu / d + 1u; }
 __device__ __forceinline__ int quot(int v, int d, unsigned m) { return d == 1 ? v : (int)__umulhi((unsigned)v, m); }
 
+// Four output channels of one voxel (w: [cin][27][4], as k_conv_s stages them), in the order
+// of k_conv_fwd; a call of its own, so that it takes no registers where it is not made.
+__device__ __noinline__ void conv_voxel(const float *in, int cin, const float4 *w, const float *bias, int d, int relu, int v,
+                                        float *out) {
+    const int n = d * d * d, x = v / (d * d), y = v / d % d, z = v % d;
+    float4 a = bias ? make_float4(bias[0], bias[1], bias[2], bias[3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int t = 0; t < cin * 27; ++t) {
+        const int o = t % 27, xx = x + o / 9 - 1, yy = y + o / 3 % 3 - 1, zz = z + o % 3 - 1;
+        if (xx < 0 || yy < 0 || zz < 0 || xx >= d || yy >= d || zz >= d) continue;
+        const float f = in[(size_t)(t / 27) * n + (xx * d + yy) * d + zz];
+        a = make_float4(fmaf(w[t].x, f, a.x), fmaf(w[t].y, f, a.y), fmaf(w[t].z, f, a.z), fmaf(w[t].w, f, a.w));
+    }
+    out[v] = relu ? fmaxf(a.x, 0.f) : a.x;
+    out[n + v] = relu ? fmaxf(a.y, 0.f) : a.y;
+    out[2 * n + v] = relu ? fmaxf(a.z, 0.f) : a.z;
+    out[3 * n + v] = relu ? fmaxf(a.w, 0.f) : a.w;
+}
+
 // The same layer, and its input gradient, with 4 output channels and ZS consecutive z
 // voxels per thread: the 4 channels' weights sit in shared memory as float32 in
 // [summed channel][27][4] order (a tap's four weights are one 16-byte broadcast), and
@@ -62,10 +81,11 @@ __device__ __forceinline__ int quot(int v, int d, unsigned m) { return d == 1 ? 
 // of one per row behind its bounds test (the four layers of two side-15 maps 490 -> 150
 // us, of 16 maps 460 -> 290).  Sums in the order of k_conv_fwd (bias, then channel,
 // then tap) and of k_conv_bwd_data (channel, then tap); a tap off the grid adds +-0, so
-// results are the same bits for finite weights.  (One that is not finite gives NaN at the
-// border, where k_conv_fwd has none.  Blocks that test their weights and take a loop of
-// their own were measured: the registers of either form cost 32 -> 32 channels, 16 maps
-// of side 15, 119 -> 130 to 152 us.)
+// results are the same bits for finite weights.  Forward, a voxel whose sums are not
+// finite is summed again by conv_voxel, which leaves such taps out as k_conv_fwd does (32
+// -> 32 channels, 16 maps of side 15: 119.5 and 121.5 us, side 18 234 and 216).  Backward a
+// weight that is not finite gives NaN at the border, where k_conv_bwd_data has none: that
+// kernel's registers would cost its layers up to 30 % (side 15 76 -> 99 us).
 // BWD: the sums run over the layer's output channels (their gradient masked where a
 // ReLU let nothing through) and the taps are mirrored.
 // SPL: a block's warps share 32 threads' voxels and sum nin / SPL channels each (added
@@ -135,6 +155,7 @@ __global__ void __launch_bounds__(128) k_conv_s(const float *in, const float *ma
             }
         }
     }
+    unsigned odd = 0u;   // voxels whose sums are not finite
     if (SPL > 1) {
         static_assert(SPL == 1 || ZS == 1, "split channels: one voxel per thread");
         __shared__ float part[SPL][128 / SPL][4];
@@ -154,7 +175,13 @@ __global__ void __launch_bounds__(128) k_conv_s(const float *in, const float *ma
         const size_t v = ((size_t)x * d + y) * d + z;
 #pragma unroll
         for (int j = 0; j < 4; ++j) out[(size_t)(c0 + j) * n + v] = !BWD && relu ? fmaxf(acc[i][j], 0.f) : acc[i][j];
+        if (!BWD && !(fabsf(acc[i][0]) + fabsf(acc[i][1]) + fabsf(acc[i][2]) + fabsf(acc[i][3]) <= FLT_MAX)) odd |= 1u << i;
     }
+    if constexpr (!BWD)
+#pragma unroll 1
+        for (; odd; odd &= odd - 1)
+            conv_voxel(in, nin, wsh4, bias ? bias + c0 : nullptr, d, relu, (x * d + y) * d + z0 + __ffs(odd) - 1,
+                       out + (size_t)c0 * n);
 }
 
 // Launch, or false where the weights do not fit or the channels do not group.
